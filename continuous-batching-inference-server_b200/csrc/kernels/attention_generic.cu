@@ -207,6 +207,146 @@ __global__ void paged_attention_generic_kernel(
   }
 }
 
+// The same for widths up to 128 whose keys' rows are whole 16-byte pieces: a LANE takes a key.  The kernel above spends a
+// group of shuffles and its own address arithmetic on every key, and asks for a group's values only after its scores: a few
+// dozen cached keys cost 28 us at 16 rows and 8 heads of 32 in 32-bit; this one takes 7.  Here the 32 lanes of a warp
+// find the places of 32 keys at once, each lane multiplies its key with the query (in shared memory, read by all lanes
+// together), the running maximum and sum move on once per 32 keys, and the values, whose addresses are known from the
+// start, are read row by row with the lanes over the dims, 32 / NPER rows in flight.
+template <typename TT, int NPER>
+__global__ void __launch_bounds__(128)
+paged_attention_lane_kernel(
+    const TT* q, int q_ld, const TT* kc, const TT* vc,
+    const int* block_table, int max_blocks, const int* row_seq,
+    const int* positions, TT* __restrict__ out, int out_ld, int n_rows, int n_head, int n_kv_head,
+    int hd, int ps, float scale, int window, int n_chunks, int chunk_keys, float* partial,
+    int hd_v, int v_row, const float* __restrict__ slopes, const float* __restrict__ sinks, float temp_coef,
+    int temp_every, const float* __restrict__ rates, int v_heads, float cap, int keep) {
+  constexpr int E = 16 / sizeof(TT), VB = 32 / NPER;      // elements per 16 bytes; rows of values in flight
+  __shared__ __align__(16) float q_sm[4][NPER * 32];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int wc = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  float* qs = q_sm[threadIdx.x >> 5];
+  if (wc >= n_rows * n_head * n_chunks) return;
+  const int w = wc / n_chunks, chunk = wc % n_chunks;
+  const int row = w / n_head, h = w % n_head;
+  const HeadPlace hp = head_place(h, n_head, n_kv_head, v_heads);
+  const int pos = positions[row];          // the step's tables were written before its first kernel
+  const int seq = row_seq[row];
+  if (temp_every > 0) scale *= 1.0f + temp_coef * logf((float)((pos + 1) / temp_every + 1));
+  const float slope = slopes ? slopes[h] : 0.f;
+  const float* rate = rates ? rates + h : nullptr;
+  const int* bt = block_table + (size_t)max(seq, 0) * max_blocks;
+  int kend = pos + 1;
+  int kstart = first_seen(pos, window);
+  if (n_chunks > 1) {   // this warp's share of the keys: chunks by absolute index, merged by a second kernel
+    kstart = max(kstart, chunk * chunk_keys);
+    kend = min(kend, (chunk + 1) * chunk_keys);
+  }
+  const int kfirst = n_chunks > 1 ? chunk * chunk_keys : 0;
+  int n_kept = kept_end(pos, window, keep);
+  if (n_chunks > 1) n_kept = min(n_kept, (chunk + 1) * chunk_keys);
+  n_kept = max(n_kept - kfirst, 0);
+  const int n_keys = seq < 0 ? 0 : n_kept + max(kend - kstart, 0);
+  const int ps_shift = (ps & (ps - 1)) == 0 ? 31 - __clz(ps) : -1;
+  // this lane's key of a group: its page's entry (asked for before the wait: a table of the step), then its token's place
+  auto key_at = [&](int i) { return i < n_kept ? kfirst + i : kstart + i - n_kept; };
+  auto page_of = [&](int i, int& off) {
+    const int j = key_at(min(i, n_keys - 1));
+    const int pi = ps_shift >= 0 ? j >> ps_shift : j / ps;
+    off = j - pi * ps;
+    return bt[pi];
+  };
+  int off = 0, page = n_keys > 0 ? page_of(lane, off) : 0;
+  pdl_wait();
+  if (seq < 0) {  // a padding row of a fixed-size batch
+    if (chunk == 0)
+      for (int dim = lane; dim < hd_v; dim += 32) from_f32(out[(size_t)row * out_ld + h * hd_v + dim], 0.f);
+    return;
+  }
+  if (n_chunks > 1 && n_keys <= 0) return;
+  for (int dim = lane; dim < hd; dim += 32) qs[dim] = to_f32(q[(size_t)row * q_ld + hp.query * hd + dim]);
+  __syncwarp();
+  float m = -INFINITY, l = 0.f, acc[NPER];
+#pragma unroll
+  for (int i = 0; i < NPER; ++i) acc[i] = 0.f;
+
+  for (int i0 = 0; i0 < n_keys; i0 += 32) {
+    const TT* kp = kc + (((size_t)page * n_kv_head + hp.key) * ps + off) * hd;
+    const long long v_at = (((long long)page * n_kv_head + hp.value) * ps + off) * v_row;
+    const int here = min(32, n_keys - i0);
+    // the first rows of values are on their way while the scores are taken
+    TT vv[VB][NPER];
+    auto load_values = [&](int u0) {
+#pragma unroll
+      for (int u = 0; u < VB; ++u) {
+        const TT* vp = vc + __shfl_sync(0xffffffffu, v_at, u0 + u);
+#pragma unroll
+        for (int i = 0; i < NPER; ++i) {
+          const int dim = lane + 32 * i;
+          if (dim < hd_v && u0 + u < here) vv[u][i] = vp[dim];
+          else from_f32(vv[u][i], 0.f);
+        }
+      }
+    };
+    load_values(0);
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = 0; c < hd; c += E) {
+      TT kv[E];
+      *reinterpret_cast<uint4*>(kv) = *reinterpret_cast<const uint4*>(kp + c);
+#pragma unroll
+      for (int e = 0; e < E; ++e) part[e & 3] = fmaf(qs[c + e], to_f32(kv[e]), part[e & 3]);
+    }
+    float s = ((part[0] + part[1]) + (part[2] + part[3])) * scale;
+    if (cap > 0.f) s = capped_score(s, cap);
+    if (slope != 0.f) s -= distance_bias(slope, rate, (float)(pos - key_at(min(i0 + lane, n_keys - 1))));
+    if (lane >= here) s = -INFINITY;
+    if (i0 + 32 < n_keys) page = page_of(i0 + 32 + lane, off);     // (kp and v_at have taken this group's)
+    const float m_new = fmaxf(m, warp_max(s));
+    const float corr = expf(m - m_new), p = expf(s - m_new);   // first group: exp(-inf) = 0
+    l = l * corr + warp_sum(p);
+#pragma unroll
+    for (int i = 0; i < NPER; ++i) acc[i] *= corr;
+    m = m_new;
+#pragma unroll
+    for (int u0 = 0; u0 < 32; u0 += VB) {
+      if (u0 >= here) break;
+      if (u0 > 0) load_values(u0);
+#pragma unroll
+      for (int u = 0; u < VB; ++u) {
+        const float pu = __shfl_sync(0xffffffffu, p, u0 + u);
+        if (u0 + u < here)
+#pragma unroll
+          for (int i = 0; i < NPER; ++i) acc[i] = fmaf(pu, to_f32(vv[u][i]), acc[i]);
+      }
+    }
+  }
+  if (n_chunks > 1) {
+    float* dst = partial + ((size_t)w * n_chunks + chunk) * (hd_v + 4);
+#pragma unroll
+    for (int i = 0; i < NPER; ++i) {
+      const int dim = lane + 32 * i;
+      if (dim < hd_v) dst[dim] = acc[i];
+    }
+    if (lane == 0) {
+      dst[hd_v] = m;
+      dst[hd_v + 1] = l;
+    }
+    return;
+  }
+  float inv = 1.f / l;
+  if (sinks) {      // the sink joins the denominator only: with the larger of the two as the reference
+    const float sk = sinks[h], mm = fmaxf(m, sk), keep1 = expf(m - mm);
+    inv = keep1 / fmaf(l, keep1, expf(sk - mm));
+  }
+#pragma unroll
+  for (int i = 0; i < NPER; ++i) {
+    const int dim = lane + 32 * i;
+    if (dim < hd_v) from_f32(out[(size_t)row * out_ld + h * hd_v + dim], acc[i] * inv);
+  }
+}
+
 }  // namespace cbis
 
 using namespace cbis;
@@ -255,13 +395,23 @@ static int launch_generic(const void* q, int q_ld, const void* kc, const void* v
                  (const TT*)kc, (const TT*)vc, block_table, max_blocks, row_seq, positions, (TT*)out, out_ld, n_rows, \
                  n_head, n_kv_head, hd, ps, scale, window, n_chunks, chunk_keys, partial, hd_v, v_row, slopes, sinks, \
                  temp_coef, temp_every, rates, v_heads, cap, keep)
+#define CBIS_LANE(NPER)                                                                                              \
+  e = launch_pdl(paged_attention_lane_kernel<TT, NPER>, dim3(blocks), dim3(warps * 32), 0, st, (const TT*)q, q_ld,   \
+                 (const TT*)kc, (const TT*)vc, block_table, max_blocks, row_seq, positions, (TT*)out, out_ld, n_rows, \
+                 n_head, n_kv_head, hd, ps, scale, window, n_chunks, chunk_keys, partial, hd_v, v_row, slopes, sinks, \
+                 temp_coef, temp_every, rates, v_heads, cap, keep)
   const int widest = hd > hd_v ? hd : hd_v;
-  if (widest <= 32) CBIS_LAUNCH(1);
+  const bool lanes = widest <= 128 && hd * sizeof(TT) % 16 == 0 && ((uintptr_t)kc & 15) == 0;
+  if (lanes && widest <= 32) CBIS_LANE(1);
+  else if (lanes && widest <= 64) CBIS_LANE(2);
+  else if (lanes) CBIS_LANE(4);
+  else if (widest <= 32) CBIS_LAUNCH(1);
   else if (widest <= 64) CBIS_LAUNCH(2);
   else if (widest <= 128) CBIS_LAUNCH(4);
   else if (widest <= 256) CBIS_LAUNCH(8);
   else CBIS_LAUNCH(16);
 #undef CBIS_LAUNCH
+#undef CBIS_LANE
   if (e == cudaSuccess && n_chunks > 1)
     e = launch_pdl(prefill_merge_kernel<TT, false>, dim3(n_rows), dim3(128), 0, st, (const float*)partial, positions, row_seq,
                    (TT*)out, out_ld, 0, n_head, hd_v, window, n_chunks, chunk_keys, sinks, keep);
