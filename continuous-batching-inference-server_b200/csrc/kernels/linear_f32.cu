@@ -75,7 +75,7 @@ linear_f32_kernel(const float* A, const float* __restrict__ W, const float* __re
 }
 
 // More than 16 rows with W stored [N, K] (both operands contiguous along k, 16-byte aligned): tiles of BM x BN
-// outputs, k in pieces of 32 that arrive by 16-byte cp.async in two buffers (the next piece is on its way while
+// outputs, k in pieces of 32 that arrive by 16-byte cp.async in a ring of buffers (the next pieces are on their way while
 // this one is multiplied), operands kept [row][k] in shared memory so that the copy is straight and a thread reads
 // four k of a row at once.  A thread owns the outputs (ty + 16 i, tx + 16 j) and walks k from left to right with
 // one fused multiply-add per element: the order of the kernels above and below, hence the same bits.  The tile
@@ -87,14 +87,22 @@ __device__ __forceinline__ void cp_async16_f32(void* smem, const void* gmem, boo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// Waits until at most N of the copies' groups are still on their way.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// NK_STAGES pieces are in the ring: a piece of a 32 x 32 tile is multiplied in 0.3 us, a trip to L2 takes 0.7, so with two
+// buffers a block waited most of its time (the two products of 512 rows with 256 columns, K 256 and 1,024: 55 us on average, now 29).
+constexpr int NK_STAGES = 5;
 template <int BM, int BN>
 __global__ void __launch_bounds__(256)
 linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                      int M, int N, int K, int act, int lda, int ldc) {
   constexpr int BK = 32, PITCH = BK + 4, TM = BM / 16, TN = BN / 16;
   extern __shared__ __align__(16) float nk_smem[];
-  float (*As)[BM][PITCH] = reinterpret_cast<float (*)[BM][PITCH]>(nk_smem);                      // [2][BM][PITCH]
-  float (*Ws)[BN][PITCH] = reinterpret_cast<float (*)[BN][PITCH]>(nk_smem + 2 * BM * PITCH);     // [2][BN][PITCH]
+  float (*As)[BM][PITCH] = reinterpret_cast<float (*)[BM][PITCH]>(nk_smem);                              // [NK_STAGES][BM][PITCH]
+  float (*Ws)[BN][PITCH] = reinterpret_cast<float (*)[BN][PITCH]>(nk_smem + NK_STAGES * BM * PITCH);     // [NK_STAGES][BN][PITCH]
   pdl_trigger();
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -118,22 +126,22 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-  load_w(0, 0);   // the weights do not come from the kernel before
-  pdl_wait();
-  load_a(0, 0);
-  asm volatile("cp.async.commit_group;\n" ::);
   const int n_kt = (K + BK - 1) / BK;
+  for (int kt = 0; kt < min(n_kt, NK_STAGES - 1); ++kt) load_w(kt * BK, kt);   // the weights do not come from the kernel before
+  pdl_wait();
+  for (int kt = 0; kt < NK_STAGES - 1; ++kt) {      // one group of copies a piece (the first holds the weights of all of these)
+    if (kt < n_kt) load_a(kt * BK, kt);
+    cp_async_commit();
+  }
   for (int kt = 0; kt < n_kt; ++kt) {
-    const int stage = kt & 1;
-    if (kt + 1 < n_kt) {
-      load_w((kt + 1) * BK, stage ^ 1);
-      load_a((kt + 1) * BK, stage ^ 1);
-      asm volatile("cp.async.commit_group;\n" ::);
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
+    const int stage = kt % NK_STAGES;
+    cp_async_wait<NK_STAGES - 2>();
+    __syncthreads();      // the piece is there for everyone, and everyone is done with the piece before it, whose buffer is filled next
+    if (kt + NK_STAGES - 1 < n_kt) {
+      load_w((kt + NK_STAGES - 1) * BK, (kt + NK_STAGES - 1) % NK_STAGES);
+      load_a((kt + NK_STAGES - 1) * BK, (kt + NK_STAGES - 1) % NK_STAGES);
     }
-    __syncthreads();
+    cp_async_commit();
     const int kc = min(BK, K - kt * BK);   // a multiple of 4; the sum stops at K (0 * 0 could still flip the sign of a zero)
 #pragma unroll 2
     for (int kk = 0; kk < kc; kk += 4) {
@@ -154,7 +162,6 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
           acc[i][j] = v;
         }
     }
-    __syncthreads();   // this buffer is free for the piece after the next
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -178,50 +185,82 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 // loads, all in flight at once, and every thread then walks its piece from left to right with one fused
 // multiply-add per element: the same order as the tiled kernel, hence the same bits, so that a token decoded
 // alone and the same token inside a prompt portion still agree exactly.
-constexpr int FR_KC = 256;
+// With 16-byte aligned rows (linear_f32_few_rows_kernel<true>) up to four pieces are on their way at once, the weights' since
+// before the wait for the kernel ahead: piece by piece, each a trip to L2 with nothing else to do, the products of a
+// 256-wide model's decode step took 6.7 us on average; now 4.9.
+constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4, FR_STAGES = 4;
+__device__ __forceinline__ float few_rows_walk(const float* a, const float* w, int kc, float acc) {
+  int k = 0;
+#pragma unroll 8
+  for (; k + 4 <= kc; k += 4) {
+    const float4 av = *reinterpret_cast<const float4*>(a + k), wv = *reinterpret_cast<const float4*>(w + k);
+    acc = fmaf(av.x, wv.x, acc);
+    acc = fmaf(av.y, wv.y, acc);
+    acc = fmaf(av.z, wv.z, acc);
+    acc = fmaf(av.w, wv.w, acc);
+  }
+  for (; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
+  return acc;
+}
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256)
 linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                            int M, int N, int K, int act, int lda, int ldc) {
-  __shared__ __align__(16) float As[16][FR_KC + 4];
-  __shared__ __align__(16) float Ws[16][FR_KC + 4];
+  extern __shared__ __align__(16) float fr_smem[];      // [stages][2][16][FR_PITCH]: A's piece, W's piece
   pdl_trigger();
   const int tid = threadIdx.x;
   const int m = tid & 15, c = tid >> 4, n0 = blockIdx.x * 16, n = n0 + c;
-  const bool vec = (K & 3) == 0 && (lda & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-  pdl_wait();  // A comes from the kernel before
   float acc = 0.f;
-  for (int k0 = 0; k0 < K; k0 += FR_KC) {
-    const int kc = min(FR_KC, K - k0);
-    if (vec) {
+  if constexpr (ALIGNED) {
+    const int n_p = (K + FR_KC - 1) / FR_KC, stages = min(n_p, FR_STAGES);
+    auto a_of = [&](int p) { return fr_smem + (size_t)(p % stages) * 32 * FR_PITCH; };
+    auto load = [&](int p, const float* src, int ld, int rows, float* dst) {      // 16 rows of 256: rows past the end are zeros
       for (int i = tid; i < 16 * (FR_KC / 4); i += 256) {
         const int r = i / (FR_KC / 4), k = (i % (FR_KC / 4)) * 4;
-        float4 av = make_float4(0.f, 0.f, 0.f, 0.f), wv = av;
-        if (k < kc) {
-          if (r < M) av = *reinterpret_cast<const float4*>(A + (size_t)r * lda + k0 + k);
-          if (n0 + r < N) wv = __ldg(reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * K + k0 + k));
-        }
-        *reinterpret_cast<float4*>(&As[r][k]) = av;
-        *reinterpret_cast<float4*>(&Ws[r][k]) = wv;
+        const bool valid = r < rows && p * FR_KC + k < K;
+        cp_async16_f32(dst + r * FR_PITCH + k, valid ? src + (size_t)r * ld + p * FR_KC + k : src, valid);
       }
-    } else {
-      for (int i = tid; i < 16 * FR_KC; i += 256) {
-        const int r = i / FR_KC, k = i % FR_KC;
-        As[r][k] = (k < kc && r < M) ? A[(size_t)r * lda + k0 + k] : 0.f;
-        Ws[r][k] = (k < kc && n0 + r < N) ? __ldg(W + (size_t)(n0 + r) * K + k0 + k) : 0.f;
+    };
+    const float* w0 = W + (size_t)n0 * K;
+    for (int p = 0; p < stages; ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+    const float b = bias && n < N ? bias[n] : 0.f;
+    pdl_wait();  // A comes from the kernel before
+    for (int p = 0; p < FR_STAGES; ++p) {
+      if (p < stages) load(p, A, lda, M, a_of(p));
+      cp_async_commit();
+    }
+    for (int p = 0; p < n_p; ++p) {
+      cp_async_wait<FR_STAGES - 1>();
+      __syncthreads();
+      const float* a = a_of(p);
+      acc = few_rows_walk(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
+      if (p + stages < n_p) {
+        __syncthreads();
+        load(p + stages, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+        load(p + stages, A, lda, M, a_of(p));
       }
+      cp_async_commit();
+    }
+    if (m < M && n < N) {
+      if (bias) acc += b;
+      C[(size_t)m * ldc + n] = activate(acc, act);
+    }
+    return;
+  }
+  float (*As)[FR_PITCH] = reinterpret_cast<float (*)[FR_PITCH]>(fr_smem);
+  float (*Ws)[FR_PITCH] = reinterpret_cast<float (*)[FR_PITCH]>(fr_smem + 16 * FR_PITCH);
+  pdl_wait();  // A comes from the kernel before
+  for (int k0 = 0; k0 < K; k0 += FR_KC) {
+    const int kc = min(FR_KC, K - k0);
+    for (int i = tid; i < 16 * FR_KC; i += 256) {
+      const int r = i / FR_KC, k = i % FR_KC;
+      As[r][k] = (k < kc && r < M) ? A[(size_t)r * lda + k0 + k] : 0.f;
+      Ws[r][k] = (k < kc && n0 + r < N) ? __ldg(W + (size_t)(n0 + r) * K + k0 + k) : 0.f;
     }
     __syncthreads();
     // (a piece shorter than 256 ends in zeros of A and W: adding 0 * 0 changes no bit of the sum... except the sign of
     // a zero sum, so the loop stops at the piece's end)
-    int k = 0;
-    for (; k + 4 <= kc; k += 4) {
-      const float4 av = *reinterpret_cast<const float4*>(&As[m][k]), wv = *reinterpret_cast<const float4*>(&Ws[c][k]);
-      acc = fmaf(av.x, wv.x, acc);
-      acc = fmaf(av.y, wv.y, acc);
-      acc = fmaf(av.z, wv.z, acc);
-      acc = fmaf(av.w, wv.w, acc);
-    }
-    for (; k < kc; ++k) acc = fmaf(As[m][k], Ws[c][k], acc);
+    acc = few_rows_walk(As[m], Ws[c], kc, acc);
     __syncthreads();
   }
   if (m < M && n < N) {
@@ -248,7 +287,7 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
 #define CBIS_NK(BM_, BN_)                                                                                              \
   {                                                                                                                    \
     auto kern = linear_f32_nk_kernel<BM_, BN_>;                                                                        \
-    const size_t smem = (size_t)2 * (BM_ + BN_) * 36 * sizeof(float);                                                  \
+    const size_t smem = (size_t)NK_STAGES * (BM_ + BN_) * 36 * sizeof(float);                                                  \
     if (smem > 48 * 1024) {                                                                                            \
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
       if (e != cudaSuccess) return (int)e;                                                                             \
@@ -272,8 +311,15 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
                            act, lda, ldc);
   }
   if (w_is_nk) {   // decoding: one thread per output, 16 outputs (rows) x 2 columns per warp, 8 warps per block
-    return (int)launch_pdl(linear_f32_few_rows_kernel, dim3((N + 15) / 16), dim3(256), 0, st, A, W, bias, C, M, N, K, act, lda,
-                           ldc);
+    const bool aligned = K % 4 == 0 && lda % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
+    auto kern = aligned ? linear_f32_few_rows_kernel<true> : linear_f32_few_rows_kernel<false>;
+    const int pieces = (K + FR_KC - 1) / FR_KC, stages = !aligned ? 1 : (pieces < FR_STAGES ? pieces : FR_STAGES);
+    const size_t smem = (size_t)stages * 32 * FR_PITCH * sizeof(float);
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return (int)e;
+    }
+    return (int)launch_pdl(kern, dim3((N + 15) / 16), dim3(256), smem, st, A, W, bias, C, M, N, K, act, lda, ldc);
   }
   dim3 grid((N + 63) / 64, (M + 15) / 16);
   return (int)launch_pdl(linear_f32_kernel<16, 64, 16, 1, 4>, grid, dim3(256), 0, st, A, W, bias, C, M, N, K, w_is_nk,
