@@ -129,6 +129,9 @@ class ModelRunner:
         self.max_shape_graphs = 24
         self.shape_graph_after = int(os.environ.get("CBIS_SHAPE_GRAPH_AFTER", "8"))
         self.shape_graph_min_host_s = 1e-3
+        # ... and, whatever a step costs the host, once its launches have cost as much as a capture does: a step of the
+        # reference's sizes (0.7 ms of launches around 0.25 ms of kernels) after some ninety times
+        self.shape_graph_capture_s = 60e-3
         self._shape_seen: Dict[tuple, int] = {}
         self._shape_graphs: "OrderedDict[tuple, tuple]" = OrderedDict()
         self.shape_captures = self.shape_replays = 0
@@ -420,7 +423,8 @@ class ModelRunner:
         """Replays the graph of this step's shape, captures it if the shape has come often enough and issuing its
         launches one by one costs the host a millisecond or more (a capture stalls the engine for tens of
         milliseconds: for a small model that is a hundred steps, and its steps cost the host little anyway), or
-        returns None (the caller then runs the step launch by launch)."""
+        returns None (the caller then runs the step launch by launch).  A cheaper shape is captured once its launches have
+        cost the host what the capture will."""
         have = self._shape_graphs.get(shape)
         if have is not None:
             self._shape_graphs.move_to_end(shape)
@@ -434,7 +438,8 @@ class ModelRunner:
             self._shape_seen.clear()
         seen = self._shape_seen.setdefault(shape, [0, 0.0])      # [times seen, host seconds of the last launch-by-launch run]
         seen[0] += 1
-        if seen[0] < self.shape_graph_after or seen[1] < self.shape_graph_min_host_s:
+        if seen[0] < self.shape_graph_after or (seen[1] < self.shape_graph_min_host_s
+                                                and seen[0] * seen[1] < self.shape_graph_capture_s):
             return None
         ctx = self.build_context(entries, fixed_shapes=True)
         # The step itself runs ONCE, launch by launch, with the launches the graph will hold; the capture that
