@@ -313,7 +313,7 @@ def raise_if_kernel_errors(device="cuda") -> None:
             flag.zero_()
             _tc_pending.pop(key, None)      # a copy of the flag asked for earlier would report the same event again
             raise KernelError(f"a bounded wait inside a TMA kernel ran out (code {code}: 1-6 and 21-24 the tcgen05 "
-                              f"product, 11-19 the prefill attention, 31-34 the persistent decode kernel); the step's "
+                              f"product, 11-19 the prefill attention, 31-34 the persistent decode kernel, 51-56 the routed feed-forward); the step's "
                               f"results are invalid")
 
 
@@ -339,7 +339,7 @@ def poll_kernel_errors(device="cuda") -> None:
             _tc_pending.pop(key, None)
             flag.zero_()
             raise KernelError(f"a bounded wait inside a TMA kernel ran out (code {code}: 1-6 and 21-24 the tcgen05 "
-                              f"product, 11-19 the prefill attention, 31-34 the persistent decode kernel); the results "
+                              f"product, 11-19 the prefill attention, 31-34 the persistent decode kernel, 51-56 the routed feed-forward); the results "
                               f"of a recent step are invalid")
     else:
         host, event = torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event()
@@ -1447,7 +1447,7 @@ ROUTED_TILES_FROM = 33     # rows from which the routed feed-forward sorts its r
 def routed_tiles_takes(h, gate_up, down) -> bool:
     """Whether ``routed_tiles`` takes these rows: bfloat16, enough of them, sizes in steps of 8, aligned."""
     W, F = gate_up.shape[2], down.shape[2]
-    return (h.dtype == torch.bfloat16 and h.shape[0] >= ROUTED_TILES_FROM and W % 8 == 0 and F % 8 == 0
+    return (USE_TCGEN05 and h.dtype == torch.bfloat16 and h.shape[0] >= ROUTED_TILES_FROM and W % 8 == 0 and F % 8 == 0
             and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0 and gate_up.shape[0] <= 4096)
 
 
@@ -1460,8 +1460,8 @@ def _routed_plan_ints(pairs: int, experts: int) -> int:
 def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accumulate=False, identity: int = 0,
                  limit: float = 0.0, beta: float = 1.0, shift: float = 0.0):
     """The routed feed-forward for many rows of bfloat16: the (row, choice) pairs are sorted by expert on the device, an
-    expert's pairs run in tiles of 128 rows on the tensor cores (gate and up with the gated activation in one kernel,
-    then down), and a row's choices are summed in their order.  ``out`` 32-bit ``[rows, width]``, overwritten or, with
+    expert's pairs run in tiles of 128 rows on the tensor cores (TMA + tcgen05; gate and up with the gated activation in one
+    kernel, then down), and a row's choices are summed in their order.  ``out`` 32-bit ``[rows, width]``, overwritten or, with
     ``accumulate``, added to.  Nothing is read back to the host: it can be captured.  ``identity``: how many choices beyond
     the experts are identity experts (the row itself times the weight); ``limit``, ``beta``, ``shift``: as in ``gate_mul``."""
     _need_cuda(h, gate_up, down, ids, weights, out)
@@ -1472,13 +1472,14 @@ def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accu
     assert out.dtype == torch.float32 and out.shape == (rows, W) and out.stride(1) == 1
     plan = torch.empty(int(_routed_plan_ints(rows * top, E)), dtype=torch.int32, device=h.device)
     hidden = torch.empty((rows * top, F), dtype=torch.bfloat16, device=h.device)
-    y = torch.empty((rows * top, W), dtype=torch.float32, device=h.device) if (top > 1 or accumulate or identity) else None
+    x = torch.empty((rows * top, W), dtype=torch.bfloat16, device=h.device)
+    y = torch.empty((rows * top, W), dtype=torch.float32, device=h.device)
     st = kernels().cbis_routed_tiles(_ptr(h), c_int(h.stride(0)), _ptr(gate_up), _ptr(down), _ptr(ids), _ptr(weights),
-                                     _ptr(plan), _ptr(hidden), _ptr(y), _ptr(out), c_int(out.stride(0)), c_int(rows),
+                                     _ptr(plan), _ptr(x), _ptr(hidden), _ptr(y), _ptr(out), c_int(out.stride(0)), c_int(rows),
                                      c_int(W), c_int(F), c_int(E), c_int(top), c_int(ACT[act]),
-                                     c_int(1 if weight_on_input else 0), c_int(1 if accumulate else 0), _stream(), c_int(identity),
-                                     c_float(limit), c_float(beta), c_float(shift))
-    _check(st, "routed_tiles", f"rows={rows} width={W} inner={F} experts={E} top={top}", launches=4 if y is not None else 3)
+                                     c_int(1 if weight_on_input else 0), c_int(1 if accumulate else 0), _stream(),
+                                     c_float(limit), c_float(beta), c_float(shift), _ptr(tcgen05_error_flag(h.device)))
+    _check(st, "routed_tiles", f"rows={rows} width={W} inner={F} experts={E} top={top}", launches=5)
 
 
 def linear_residual(x, w_nk, residual) -> bool:
