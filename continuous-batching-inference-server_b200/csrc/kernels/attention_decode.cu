@@ -249,6 +249,15 @@ paged_decode_bf16_kernel(const __nv_bfloat16* qkv, int ld, int k_off, int v_off,
 // ---------------------------------------------------------------------------------------------
 // The fast form for head sizes 64 and 128 and pages of a multiple of 16 keys: decode_tc_item of
 // attention_decode_tc.cuh, one block of four warps per (row, head, split).
+//
+// nsplit > 0: every row is cut so many ways, block (row, head, split).  nsplit == 0: the rows of a step are rarely of one
+// length, and blocks of unlike length leave SMs idle while the longest ones finish: the rows are then cut by their own
+// lengths, into pieces of about one size, as a plan says that decode_plan_kernel has made from the positions (a captured
+// step reads them from memory) before the step's first attention.  Block x takes piece x / n_head for head x % n_head; the
+// grid holds as many blocks as there can be pieces, and those left over end at once.  A layer's time, even cut -> plan: 64 rows
+// of 120 to 1,400 keys, 16 heads of 128, 75 -> 63 us (their bytes take 61); 23 rows of 90 to 1,100, 52 -> 33 us; 37 rows of
+// 32 to 1,000, 25 heads of 64, 32 -> 28 us; 8 rows of 1,024 to 2,000, 24 -> 22 us.  Several rounds of shorter pieces were
+// slower: a piece costs its first trip to memory and its share of the merge.
 // ---------------------------------------------------------------------------------------------
 template <int HD, bool BIAS, bool EXT>
 __global__ void __launch_bounds__(DEC_WARPS * 32, 4)   // 128 registers: four blocks per SM
@@ -257,12 +266,92 @@ paged_decode_tc_kernel(const __nv_bfloat16* qkv, int ld, int k_off, int v_off, _
                        const int* slot_mapping, __nv_bfloat16* __restrict__ out, int out_ld, float* part,
                        unsigned int* counters, int n_head, int n_kv_head, int ps, float scale, int window,
                        int nsplit, const float* __restrict__ sinks, const float* __restrict__ slopes,
-                       const float* __restrict__ rates, float cap, int keep) {
+                       const float* __restrict__ rates, float cap, int keep, const DecodePiece* plan) {
   __shared__ DecodeTcShared<HD> sm;
+  constexpr int TPW = HD <= 64 ? 2 : 1;
   pdl_trigger();
-  decode_tc_item<HD, true, (HD <= 64 ? 2 : 1), BIAS, EXT>(qkv, ld, k_off, v_off, kc, vc, block_table, max_blocks, row_seq, positions, slot_mapping, out,
-                           out_ld, part, counters, n_head, n_kv_head, ps, scale, window, nsplit, blockIdx.x, blockIdx.y,
-                           blockIdx.z, threadIdx.x, sm, 0, sinks, slopes, rates, cap, keep);
+  int row = blockIdx.x, h = blockIdx.y, split = blockIdx.z, seq, pos;
+  size_t part_at = ((size_t)row * n_head + h) * nsplit;
+  if (nsplit == 0) {
+    h = blockIdx.x % n_head;
+    const DecodePiece p = plan[blockIdx.x / n_head];
+    if (p.what < 0) return;      // (the kernel ends with the blocks that have a piece: those wait for the kernels ahead)
+    row = p.what & (PLAN_MAX_ROWS - 1);
+    split = (p.what >> 12) & 31;
+    nsplit = (p.what >> 17) + 1;
+    part_at = (size_t)p.before * n_head + (size_t)h * nsplit;
+    seq = p.seq;
+    pos = p.pos;
+  } else {
+    seq = row_seq[row];
+    pos = positions[row];
+  }
+  decode_tc_item<HD, true, TPW, BIAS, EXT>(qkv, ld, k_off, v_off, kc, vc, block_table, max_blocks, seq, pos, slot_mapping, out,
+                           out_ld, part, counters, n_head, n_kv_head, ps, scale, window, nsplit, part_at, row, h,
+                           split, threadIdx.x, sm, 0, sinks, slopes, rates, cap, keep);
+}
+
+// The plan of a step's decoding rows for one window: how many keys a piece holds, then every row's pieces, the longest
+// pieces first (blocks start in this order, so the short ones fill the gaps at the end).  A head's pieces: `fit` at most
+// where the rows leave room for that (one round of blocks over the SMs: a piece more than they hold would cost a second
+// round), else about `fit` in all.  No piece is shorter than `round` keys and no row has more than 32.
+// One block; it lets its successor start only when it ends: an attention kernel reads its plan before it waits for
+// the kernels ahead.
+constexpr int PLAN_THREADS = 256;
+__global__ void __launch_bounds__(PLAN_THREADS)
+decode_plan_kernel(const int* row_seq, const int* positions, int rows, int window, int keep, int fit, int round, DecodePiece* plan,
+                   int most) {
+  __shared__ long long s_total;
+  __shared__ int s_longest, s_keys;
+  extern __shared__ int s_rows[];                 // [rows] pieces, [rows] keys of a piece
+  int *n_of = s_rows, *len_of = s_rows + rows;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    s_total = 0;
+    s_longest = 0;
+  }
+  __syncthreads();
+  long long total = 0;
+  int longest = 0;
+  for (int r = tid; r < rows; r += PLAN_THREADS) {
+    const int span = row_seq[r] >= 0 ? decode_span(positions[r], window, keep) : 0;
+    len_of[r] = span;
+    total += span;
+    longest = max(longest, span);
+  }
+  atomicAdd(reinterpret_cast<unsigned long long*>(&s_total), (unsigned long long)total);
+  atomicMax(&s_longest, longest);
+  __syncthreads();
+  if (tid < 32) {
+    // lane i tries i rounds more than an even share: the first that fits
+    const long long even = max((s_total + fit - 1) / fit, (long long)(s_longest + 31) / 32);
+    const int keys0 = (int)((even + round - 1) / round) * round;
+    const int keys = max(keys0, round) + lane * round;
+    int n = 0;
+    for (int r = 0; r < rows; ++r) n += max((len_of[r] + keys - 1) / keys, 1);
+    const unsigned ok = __ballot_sync(0xffffffffu, n <= fit);
+    const int pick = rows > fit ? 0 : (ok ? __ffs(ok) - 1 : 31);
+    if (lane == pick) s_keys = keys;
+  }
+  __syncthreads();
+  for (int r = tid; r < rows; r += PLAN_THREADS) n_of[r] = max((len_of[r] + s_keys - 1) / s_keys, 1);
+  __syncthreads();
+  for (int r = tid; r < rows; r += PLAN_THREADS) len_of[r] = (len_of[r] + n_of[r] - 1) / n_of[r];
+  __syncthreads();
+  // the plan's memory may be an earlier kernel's until that has finished: written only after the wait
+  pdl_wait();
+  // every row's place: the pieces of the rows whose pieces are longer (equal ones in the rows' order)
+  int all = 0;
+  for (int r = tid; r < rows; r += PLAN_THREADS) {
+    int before = 0;
+    for (int o = 0; o < rows; ++o)
+      if (len_of[o] > len_of[r] || (len_of[o] == len_of[r] && o < r)) before += n_of[o];
+    for (int i = 0; i < n_of[r] && before + i < most; ++i) 
+      plan[before + i] = DecodePiece{r | i << 12 | (n_of[r] - 1) << 17, before, row_seq[r], positions[r]};
+  }
+  for (int o = 0; o < rows; ++o) all += n_of[o];
+  for (int i = all + tid; i < most; i += PLAN_THREADS) plan[i] = DecodePiece{-1, 0, -1, 0};
+  __threadfence();
 }
 
 // After a decode step whose next tokens were chosen on the device: the chosen token becomes the
@@ -311,13 +400,16 @@ CBIS_EXPORT long long cbis_paged_decode_scratch_floats(int rows, int n_head, int
 
 // qkv: this step's projections [rows, ld], queries at column 0.  k_off/v_off >= 0: take the current
 // token's key/value from qkv and store them at slot_mapping[row]; < 0: the cache holds them already.
+// nsplit 0 (the fast form only): the rows' keys are cut as `plan` says (cbis_decode_plan, `most_pieces` entries); `part` then
+// holds n_head * most_pieces results of hd + 2 floats.
 CBIS_EXPORT int cbis_paged_decode_bf16(const void* qkv, int ld, int k_off, int v_off, void* kc, void* vc,
                                        const int* block_table, int max_blocks, const int* row_seq,
                                        const int* positions, const int* slot_mapping, void* out, int out_ld,
                                        float* part, unsigned int* counters, int rows, int n_head, int n_kv_head,
                                        int hd, int ps, float scale, int window, int nsplit, void* stream, int hdv,
                                        int v_row, const float* slopes, const float* sinks, float temp_coef,
-                                       int temp_every, const float* rates, int v_heads, float cap, int keep) {
+                                       int temp_every, const float* rates, int v_heads, float cap, int keep, const void* plan,
+                                       int most_pieces) {
   if (rows <= 0) return CBIS_OK;
   // hdv (0: the keys' width, values in pages of their own): the values' width.  With values of another width or in
   // the keys' rows, a linear bias or a temperature the lane-group form runs whatever the head size; a sink (it joins
@@ -329,12 +421,12 @@ CBIS_EXPORT int cbis_paged_decode_bf16(const void* qkv, int ld, int k_off, int v
   if (keep < 0) return CBIS_ERR_BAD_SIZE;
   if (v_heads != 1 && (v_heads != n_kv_head || n_head % v_heads)) return CBIS_ERR_BAD_SIZE;
   if (hdv > 256 || hdv % 8 || v_row < hdv || v_row % 8) return CBIS_ERR_BAD_SIZE;
-  if (hd <= 0 || hd > 256 || hd % 8 || ps <= 0 || n_head <= 0 || n_kv_head <= 0 || (n_head / v_heads) % n_kv_head || nsplit < 1 || nsplit > 32)
+  if (hd <= 0 || hd > 256 || hd % 8 || ps <= 0 || n_head <= 0 || n_kv_head <= 0 || (n_head / v_heads) % n_kv_head || nsplit < 0 || nsplit > 32)
     return CBIS_ERR_BAD_SIZE;
   if (ld % 8 || out_ld % 8 || (k_off >= 0 && (k_off % 8 || v_off % 8)) || ((uintptr_t)qkv & 15) || ((uintptr_t)kc & 15) ||
       ((uintptr_t)vc & 15))
     return CBIS_ERR_ALIGNMENT;
-  if (nsplit > 1 && (part == nullptr || counters == nullptr)) return CBIS_ERR_BAD_SIZE;
+  if (nsplit != 1 && (part == nullptr || counters == nullptr)) return CBIS_ERR_BAD_SIZE;
   cudaStream_t st = (cudaStream_t)stream;
   dim3 grid(rows, n_head, nsplit);
   const int chunks = (hd > hdv ? hd : hdv) / 8;
@@ -344,11 +436,16 @@ CBIS_EXPORT int cbis_paged_decode_bf16(const void* qkv, int ld, int k_off, int v
                                     : (ext ? paged_decode_tc_kernel<128, false, true> : paged_decode_tc_kernel<128, false, false>))
                           : (slopes ? paged_decode_tc_kernel<64, true, false>
                                     : (ext ? paged_decode_tc_kernel<64, false, true> : paged_decode_tc_kernel<64, false, false>));
+    if (nsplit == 0) {
+      if (plan == nullptr || ((uintptr_t)plan & 15) || most_pieces < rows || (long long)n_head * most_pieces > 0x7fffffffLL) return CBIS_ERR_BAD_SIZE;
+      grid = dim3((unsigned)(n_head * most_pieces));
+    }
     return (int)launch_pdl(kern, grid, dim3(DEC_WARPS * 32), 0, st, (const __nv_bfloat16*)qkv, ld, k_off,
                      v_off, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, block_table, max_blocks, row_seq, positions,
                      slot_mapping, (__nv_bfloat16*)out, out_ld, part, counters, n_head, n_kv_head, ps, scale, window,
-                     nsplit, sinks, slopes, rates, cap, keep);
+                     nsplit, sinks, slopes, rates, cap, keep, (const DecodePiece*)plan);
   }
+  if (nsplit == 0) return CBIS_ERR_BAD_SIZE;
 #define CBIS_DEC(LPK)                                                                                             \
   e = launch_pdl(paged_decode_bf16_kernel<LPK>, grid, dim3(DEC_WARPS * 32), 0, st, (const __nv_bfloat16*)qkv, ld, \
                  k_off, v_off, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, block_table, max_blocks, row_seq, positions, \
@@ -361,6 +458,17 @@ CBIS_EXPORT int cbis_paged_decode_bf16(const void* qkv, int ld, int k_off, int v
   else CBIS_DEC(32);
 #undef CBIS_DEC
   return (int)e;
+}
+
+// The plan for cbis_paged_decode_bf16 with nsplit 0: `plan` takes `most` entries of 16 bytes, of which at most
+// rows + fit are pieces (most >= that, or >= rows times the most pieces a row can have).  rows <= PLAN_MAX_ROWS.
+CBIS_EXPORT int cbis_decode_plan(const int* row_seq, const int* positions, int rows, int window, int keep, int fit, int round,
+                                 void* plan, int most, void* stream) {
+  if (rows <= 0) return CBIS_OK;
+  if (rows > PLAN_MAX_ROWS || fit < 1 || round < 16 || round % 16 || most < rows || keep < 0) return CBIS_ERR_BAD_SIZE;
+  if ((uintptr_t)plan & 15) return CBIS_ERR_ALIGNMENT;
+  return (int)launch_pdl(decode_plan_kernel, dim3(1), dim3(PLAN_THREADS), (size_t)rows * 8, (cudaStream_t)stream, row_seq,
+                         positions, rows, window, keep, fit, round, (DecodePiece*)plan, most);
 }
 
 CBIS_EXPORT int cbis_decode_advance(int* tokens, int* positions, int* seg_start, int* seg_ctx, const int* sampled,

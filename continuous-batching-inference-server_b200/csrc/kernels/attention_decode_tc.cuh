@@ -62,6 +62,21 @@ __device__ __forceinline__ void mma_16816(float* c, uint32_t a0, uint32_t a1, ui
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// One entry of a decode step's plan (decode_plan_kernel in attention_decode.cu): a piece of one row's keys, in 16 bytes, with
+// the row's request and position, so that a block has all it needs to know in one load.
+struct __align__(16) DecodePiece {
+  int what;                // row | piece << 12 | (the row's pieces - 1) << 17; -1: no piece
+  int before;              // pieces of the rows before this one: where its partial results start
+  int seq, pos;
+};
+constexpr int PLAN_MAX_ROWS = 4096;
+// Keys along the numbering of decode_tc_item that the query at `pos` walks over.
+__device__ __forceinline__ int decode_span(int pos, int window, int keep) {
+  const int first_tile = first_seen(pos, window) >> 4;
+  const int nk = min((kept_end(pos, window, keep) + 15) >> 4, first_tile);
+  return pos + 1 - ((first_tile - nk) << 4);
+}
+
 // Shared memory of one group of four warps.
 template <int HD>
 struct DecodeTcShared {
@@ -73,10 +88,11 @@ struct DecodeTcShared {
   int is_last;
 };
 
-// One (row, head, split) by a group of DEC_WARPS warps: `tid` is the thread's index in the group (0..127), `bar` the
+// One (row, head, split) of request `seq` (negative: a padding row) at position `pos` by a group of DEC_WARPS warps: `tid` is the thread's index in the group (0..127), `bar` the
 // hardware barrier the group meets at.  STANDALONE: the group is a block launched for this alone, which waits for
 // the kernels ahead (programmatic dependent launch) after it has fetched what they do not write.  The group's
-// threads must have met (group_sync) between two calls, since the calls share `sm`.
+// threads must have met (group_sync) between two calls, since the calls share `sm`.  The nsplit partial results of a (row,
+// head) lie one after the other in `part`, the first at place `part_at` (in results, not in floats).
 //
 // EXT: a cap on the scaled scores, and first keys that stay visible behind a window (keep).  The tiles are then numbered
 // along what the row sees, the nk tiles that hold kept keys first: tiles, ks, ke and kend are such numbers, `real_tile`
@@ -84,10 +100,10 @@ struct DecodeTcShared {
 template <int HD, bool STANDALONE, int TPW = 1, bool BIAS = false, bool EXT = false>
 __device__ __forceinline__ void decode_tc_item(const __nv_bfloat16* qkv, int ld, int k_off, int v_off, __nv_bfloat16* kc,
                                                __nv_bfloat16* vc, const int* block_table, int max_blocks,
-                                               const int* row_seq, const int* positions, const int* slot_mapping,
+                                               int seq, int pos, const int* slot_mapping,
                                                __nv_bfloat16* out, int out_ld, float* part, unsigned int* counters,
                                                int n_head, int n_kv_head, int ps, float scale, int window, int nsplit,
-                                               int row, int h, int split, int tid, DecodeTcShared<HD>& sm, int bar,
+                                               size_t part_at, int row, int h, int split, int tid, DecodeTcShared<HD>& sm, int bar,
                                                const float* __restrict__ sinks = nullptr,
                                                const float* __restrict__ slopes = nullptr,
                                                const float* __restrict__ rates = nullptr, float cap = 0.f,
@@ -105,7 +121,6 @@ __device__ __forceinline__ void decode_tc_item(const __nv_bfloat16* qkv, int ld,
   // cached keys and values of earlier positions by earlier steps: they are read, and this warp's first
   // tile is fetched, while the kernels ahead (the projection of this step's q, k, v) still run.
   const int lane = tid & 31, warp = tid >> 5;
-  const int seq = row_seq[row];
   if (seq < 0) {  // a padding row of a fixed-size batch
     if (STANDALONE) pdl_wait();
     if (split == 0)
@@ -113,7 +128,6 @@ __device__ __forceinline__ void decode_tc_item(const __nv_bfloat16* qkv, int ld,
     return;
   }
   const int hk = h / (n_head / n_kv_head);
-  const int pos = positions[row];
   const int kstart = first_seen(pos, window);
   const int kept = EXT ? kept_end(pos, window, keep) : 0;
   const int first_tile = kstart >> 4;
@@ -311,7 +325,7 @@ __device__ __forceinline__ void decode_tc_item(const __nv_bfloat16* qkv, int ld,
     if (nsplit == 1) {
       out[(size_t)row * out_ld + h * HD + tt] = __float2bfloat16_rn(v * keep1 / L);
     } else {
-      float* p = part + (((size_t)row * n_head + h) * nsplit + split) * (HD + 2);
+      float* p = part + (part_at + split) * (HD + 2);
       p[tt] = v;
       if (tt == 0) {
         p[HD] = M;
@@ -327,7 +341,7 @@ __device__ __forceinline__ void decode_tc_item(const __nv_bfloat16* qkv, int ld,
   if (!sm.is_last) return;
   __threadfence();
   // weights of the splits first (one thread per split), then every thread sums its dims over the splits
-  const float* p = part + ((size_t)row * n_head + h) * nsplit * (HD + 2);
+  const float* p = part + part_at * (HD + 2);
   if (warp == 0) {
     const float ms = lane < nsplit ? __ldcg(p + (size_t)lane * (HD + 2) + HD) : -INFINITY;
     const float ls = lane < nsplit ? __ldcg(p + (size_t)lane * (HD + 2) + HD + 1) : 0.f;

@@ -469,9 +469,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
       const int n_items = p.M * p.n_head * p.nsplit, n_groups = gridDim.x * (CONSUMER_WARPS / DEC_WARPS);
       for (int item = blockIdx.x * (CONSUMER_WARPS / DEC_WARPS) + group; item < n_items; item += n_groups) {
         const int split = item % p.nsplit, rh = item / p.nsplit;
-        decode_tc_item<HD, false>(p.qkv, n_qkv, p.d_q, p.d_q + p.d_kv, L.kc, L.vc, p.block_table, p.max_blocks, p.row_seq,
-                                  p.positions, p.slot_mapping, p.attn, p.d_q, p.part, p.counters, p.n_head, p.n_kv_head,
-                                  p.ps, p.scale, p.window, p.nsplit, rh / p.n_head, rh % p.n_head, split, gtid, att[group],
+        decode_tc_item<HD, false>(p.qkv, n_qkv, p.d_q, p.d_q + p.d_kv, L.kc, L.vc, p.block_table, p.max_blocks,
+                                  p.row_seq[rh / p.n_head], p.positions[rh / p.n_head], p.slot_mapping, p.attn, p.d_q, p.part, p.counters, p.n_head, p.n_kv_head,
+                                  p.ps, p.scale, p.window, p.nsplit, (size_t)rh * p.nsplit, rh / p.n_head, rh % p.n_head, split, gtid, att[group],
                                   BAR_GROUP0 + group);
         group_sync(BAR_GROUP0 + group, DEC_WARPS * 32);
       }

@@ -52,6 +52,24 @@ def _general_chunks(ctx, n_head, rows, hd):
     return chunks, partial
 
 
+def _decode_cut(ctx, v_pages, n_head, hd, vd, ps, window, extra):
+    """How the decode kernel cuts the decoding rows' keys, and the scratch memory for that: (splits, plan, scratch,
+    counters).  Where the kernel can, by the rows' own lengths, in pieces of about one size; the plan of that is made once
+    for all layers of the step that cut alike."""
+    nd, limit = ctx.n_decode, ctx.ctx_limit
+    # (a single row is cut evenly in any case; its pieces need no plan, whose lookup cost 1.5 us a layer)
+    if 1 < nd <= 4096 and ops.decode_in_pieces(v_pages, hd, ps, **extra):
+        key = ("decode_plan", n_head, hd, window, extra.get("keep", 0))
+        plan = ctx.shared.get(key)
+        if plan is None:
+            plan = ctx.shared[key] = ops.decode_plan(ctx.row_seq, ctx.positions, nd, n_head, limit, hd, window, extra.get("keep", 0))
+        return (0, plan) + ctx.decode_scratch(n_head * plan.shape[0] * (hd + 2), nd * n_head)
+    nsplit = ops.decode_splits(nd, n_head, limit)
+    if nsplit == 1:
+        return 1, None, None, None
+    return (nsplit, None) + ctx.decode_scratch(ops.decode_scratch_floats(nd, n_head, vd, nsplit), nd * n_head)
+
+
 def _extended(ctx, mixer, qkv, cache, view, out, k_pages, v_pages, k_off, v_off, vd, slopes, sinks, q_temp,
               rates, v_heads=1, done=0, cap=0.0, keep=0) -> int:
     """Attention with values of their own width, a distance bias, a sink, a query temperature, a cap on the scores or kept
@@ -73,13 +91,10 @@ def _extended(ctx, mixer, qkv, cache, view, out, k_pages, v_pages, k_off, v_off,
     tiled = by8 and T > nd and max(hd, vd) <= 128 and ps & (ps - 1) == 0 and ops.USE_TILED_EXTENDED
     first = nd if fast_decode else done     # rows from here on have their keys and values stored by the cache-write kernel
     if fast_decode:
-        nsplit = ops.decode_splits(nd, n_head, ctx.ctx_limit)
-        scratch = counters = None
-        if nsplit > 1:
-            scratch, counters = ctx.decode_scratch(ops.decode_scratch_floats(nd, n_head, vd, nsplit), nd * n_head)
+        nsplit, plan, scratch, counters = _decode_cut(ctx, v_pages, n_head, hd, vd, ps, mixer.window, extra)
         ops.paged_decode_bf16(qkv[:nd], k_off if mixer.own_kv else -1, v_off if mixer.own_kv else -1, k_pages, v_pages,
                               view.block_table, ctx.row_seq, ctx.positions, view.slot_mapping, o[:nd], scratch, counters,
-                              n_head, mixer.n_kv_head, hd, ps, mixer.scale, mixer.window, nsplit, **extra)
+                              n_head, mixer.n_kv_head, hd, ps, mixer.scale, mixer.window, nsplit, plan=plan, **extra)
     if first >= T:
         return vd
     r = slice(first, T)
@@ -162,15 +177,10 @@ def _plain(ctx, mixer, qkv, cache, view, out, nd, T, hd, ps, k_pages, v_pages, k
     fast_decode = qkv.dtype == torch.bfloat16 and hd % 8 == 0 and hd <= 256 and nd > 0
     first_general = nd if fast_decode else 0
     if fast_decode:
-        limit = ctx.ctx_limit
-        nsplit = ops.decode_splits(nd, mixer.n_head, limit)
-        scratch = counters = None
-        if nsplit > 1:
-            scratch, counters = ctx.decode_scratch(ops.decode_scratch_floats(nd, mixer.n_head, hd, nsplit),
-                                                   nd * mixer.n_head)
+        nsplit, plan, scratch, counters = _decode_cut(ctx, v_pages, mixer.n_head, hd, hd, ps, mixer.window, {})
         ops.paged_decode_bf16(qkv[:nd], k_off if mixer.own_kv else -1, v_off if mixer.own_kv else -1, k_pages, v_pages,
                               view.block_table, ctx.row_seq, ctx.positions, view.slot_mapping, out[:nd], scratch, counters,
-                              mixer.n_head, mixer.n_kv_head, hd, ps, mixer.scale, mixer.window, nsplit)
+                              mixer.n_head, mixer.n_kv_head, hd, ps, mixer.scale, mixer.window, nsplit, plan=plan)
     if first_general < T:
         r = slice(first_general, T)
         if mixer.own_kv:

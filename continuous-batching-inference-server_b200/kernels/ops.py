@@ -581,10 +581,42 @@ def decode_scratch_floats(rows: int, n_head: int, head_dim: int, nsplit: int) ->
     return rows * n_head * nsplit * (head_dim + 2) if nsplit > 1 else 0
 
 
+def decode_in_pieces(v_cache, head_dim, page_size, v_head_dim=0, slopes=None, q_temp=None, rates=None, v_heads=1, cap=0.0,
+                     keep=0, sinks=None) -> bool:
+    """Whether ``paged_decode_bf16`` can cut this attention's keys by the rows' own lengths (``nsplit`` 0): what its
+    tensor-core form takes."""
+    return (head_dim in (64, 128) and page_size % 16 == 0 and (v_head_dim or head_dim) == head_dim and v_cache.shape[-1] == head_dim
+            and (slopes is None or rates is not None) and q_temp is None and v_heads == 1 and not (slopes is not None and (cap or keep)))
+
+
+def decode_plan_entries(rows: int, n_head: int, max_context: int, head_dim: int) -> int:
+    """Entries of ``decode_plan``: the most pieces the rows' keys can come in (per head)."""
+    return min(rows + max(1, 4 * 148 // n_head), rows * min(32, -(-max_context // _decode_round(head_dim))))
+
+
+def _decode_round(head_dim: int) -> int:
+    return 64 if head_dim > 64 else 128      # keys that the four warps of a block take through one round of loads
+
+
+def decode_plan(row_seq, positions, rows: int, n_head: int, max_context: int, head_dim: int, window: int = 0, keep: int = 0):
+    """How ``paged_decode_bf16`` with ``nsplit`` 0 cuts the keys of a step's first ``rows`` rows (all of them decoding, no
+    context longer than ``max_context``): int32 [entries, 4] on the device, made from the positions there.  It serves every
+    attention of the step with the same window, heads and head size.  Four blocks fit on each of the 148 SMs."""
+    _need_cuda(row_seq, positions)
+    assert row_seq.dtype == torch.int32 and positions.dtype == torch.int32 and min(row_seq.numel(), positions.numel()) >= rows
+    n = decode_plan_entries(rows, n_head, max_context, head_dim)
+    plan = torch.empty((n, 4), dtype=torch.int32, device=positions.device)
+    st = kernels().cbis_decode_plan(_ptr(row_seq), _ptr(positions), c_int(rows), c_int(window), c_int(keep),
+                                    c_int(max(1, 4 * 148 // n_head)), c_int(_decode_round(head_dim)), _ptr(plan), c_int(n), _stream())
+    _check(st, "decode_plan", f"rows={rows} heads={n_head}")
+    return plan
+
+
 def paged_decode_bf16(qkv, k_off, v_off, k_cache, v_cache, block_table, row_seq, positions, slot_mapping, out,
                       scratch, counters, n_head, n_kv_head, head_dim, page_size, scale, window, nsplit, v_head_dim=0,
-                      slopes=None, sinks=None, q_temp=None, rates=None, v_heads=1, cap: float = 0.0, keep: int = 0):
-    """Decode attention (one query per row) with the keys split ``nsplit`` ways; with ``k_off >= 0`` the
+                      slopes=None, sinks=None, q_temp=None, rates=None, v_heads=1, cap: float = 0.0, keep: int = 0, plan=None):
+    """Decode attention (one query per row) with the keys split ``nsplit`` ways, or, with ``nsplit`` 0, by the rows' lengths
+    (``plan`` from ``decode_plan``; ``scratch`` then holds n_head * plan.shape[0] * (head_dim + 2) floats); with ``k_off >= 0`` the
     current token's key/value are taken from ``qkv`` and stored into the cache by the same kernel.
     ``scratch``: ``decode_scratch_floats`` floats; ``counters``: rows*n_head int32, zero before the
     first launch (every launch leaves them zero).  ``v_head_dim``, ``slopes``, ``sinks``, ``q_temp``, ``rates``, ``v_heads``,
@@ -599,8 +631,9 @@ def paged_decode_bf16(qkv, k_off, v_off, k_cache, v_cache, block_table, row_seq,
         assert t is None or (t.dtype == torch.float32 and t.numel() == n_head)
     coef, every = q_temp if q_temp else (0.0, 0)
     _need_columns(qkv, out, n_head, v_heads, head_dim, vd)
-    if nsplit > 1:
-        assert scratch.dtype == torch.float32 and scratch.numel() >= decode_scratch_floats(rows, n_head, vd, nsplit)
+    if nsplit != 1:
+        assert scratch.dtype == torch.float32
+        assert scratch.numel() >= (decode_scratch_floats(rows, n_head, vd, nsplit) if nsplit else n_head * plan.shape[0] * (head_dim + 2))
         assert counters.dtype == torch.int32 and counters.numel() >= rows * n_head
     st = kernels().cbis_paged_decode_bf16(
         _ptr(qkv), c_int(qkv.stride(0)), c_int(k_off), c_int(v_off), _ptr(k_cache), _ptr(v_cache), _ptr(block_table),
@@ -608,7 +641,8 @@ def paged_decode_bf16(qkv, k_off, v_off, k_cache, v_cache, block_table, row_seq,
         c_int(out.stride(0)), _ptr(scratch), _ptr(counters), c_int(rows), c_int(n_head), c_int(n_kv_head),
         c_int(head_dim), c_int(page_size), c_float(scale), c_int(window), c_int(nsplit), _stream(),
         c_int(int(v_head_dim)), c_int(v_cache.shape[-1]), _ptr(slopes), _ptr(sinks), c_float(coef), c_int(int(every)),
-        _ptr(rates), c_int(v_heads), c_float(cap), c_int(keep))
+        _ptr(rates), c_int(v_heads), c_float(cap), c_int(keep), _ptr(plan),
+        c_int(0 if plan is None else plan.shape[0]))
     _check(st, "paged_decode_bf16", f"rows={rows} heads={n_head}/{n_kv_head} head_dim={head_dim} splits={nsplit}")
 
 
