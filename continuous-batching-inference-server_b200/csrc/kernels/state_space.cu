@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256)
 ssm_scan_kernel(const TT* xbc, int xbc_ld, const TT* proj, int proj_ld, int dt_off, const float* __restrict__ dt_bias,
                 const float* __restrict__ A_log, const float* __restrict__ Dskip, float* state, long long slot_stride,
                 const int* seg_slot, const int* cu_rows, float* y, int y_ld, int H, int P, int N, int G, int use_async,
-                int mode, int n_chunks, int chunk_rows, float* chunk_state, float* chunk_logdecay) {
+                int mode, int n_chunks, int chunk_rows, float* chunk_state, float* chunk_logdecay, int below_rows) {
   constexpr int NP = L * NPL;                       // the state size rounded up
   constexpr int TC = kScanTokens;
   constexpr int CB = 256 / L;                       // columns a block
@@ -154,7 +154,7 @@ ssm_scan_kernel(const TT* xbc, int xbc_ld, const TT* proj, int proj_ld, int dt_o
   const int h = blockIdx.y, s = blockIdx.z / n_chunks, chunk = blockIdx.z % n_chunks;
   const int seg_row0 = cu_rows[s], seg_rows = cu_rows[s + 1] - seg_row0;
   const int first_row = mode == 0 ? 0 : chunk * chunk_rows;
-  if (first_row >= seg_rows) return;
+  if (first_row >= seg_rows || (below_rows > 0 && seg_rows >= below_rows)) return;
   const int n_rows = mode == 0 ? seg_rows : min(chunk_rows, seg_rows - first_row);
   const bool last_piece = first_row + n_rows == seg_rows;
   if (mode == 1 && last_piece) return;          // nobody comes after it
@@ -349,7 +349,7 @@ template <typename TT>
 static int launch_scan(const void* xbc, int xbc_ld, const void* proj, int proj_ld, int dt_off, const float* dt_bias,
                        const float* A_log, const float* D, float* state, long long slot_stride, const int* seg_slot,
                        const int* cu_rows, float* y, int y_ld, int S, int H, int P, int N, int G, int mode, int n_chunks,
-                       int chunk_rows, float* chunk_state, float* chunk_logdecay, cudaStream_t st) {
+                       int chunk_rows, float* chunk_state, float* chunk_logdecay, int below_rows, cudaStream_t st) {
   // lanes a column: 8, or 16 while the warps (segments x heads x columns x lanes / 32) would not give every SM its
   // sixteen.  Not 32: the blocks of one long prompt (every one walks the whole prompt) must all run at once, and 512
   // blocks of 33 KB of shared memory do not (measured: 32 lanes took twice as long as 8).
@@ -363,7 +363,7 @@ static int launch_scan(const void* xbc, int xbc_ld, const void* proj, int proj_l
   return (int)launch_pdl(ssm_scan_kernel<TT, NPL, LL>, dim3((P + 256 / LL - 1) / (256 / LL), H, S * n_chunks), dim3(256), 0, st, \
                          (const TT*)xbc, xbc_ld, (const TT*)proj, proj_ld, dt_off, dt_bias, A_log, D, state, slot_stride, \
                          seg_slot, cu_rows, y, y_ld, H, P, N, G, use_async, mode, n_chunks, chunk_rows, chunk_state, \
-                         chunk_logdecay)
+                         chunk_logdecay, below_rows)
   if (L == 16) {
     if (N <= 64) CBIS_SCAN(4, 16);
     if (N <= 128) CBIS_SCAN(8, 16);
@@ -432,12 +432,14 @@ CBIS_EXPORT int cbis_conv_state_update(const void* in, int in_ld, int c0, float*
 
 // xbc [T, xbc_ld]: x | B | C after the convolution (compute type); proj [T, proj_ld] holds the raw step sizes at
 // columns dt_off .. dt_off + H - 1; y [T, y_ld] 32-bit; state: H * P * N floats at `state + slot * slot_stride`.
+// below_rows > 0: only the segments of fewer rows are walked (the others are cbis_ssm_chunks's).
 CBIS_EXPORT int cbis_ssm_scan(const void* xbc, int xbc_ld, const void* proj, int proj_ld, int dt_off,
                               const float* dt_bias, const float* A_log, const float* D, float* state,
                               long long slot_stride, const int* seg_slot, const int* cu_rows, float* y, int y_ld,
                               int n_segments, int H, int P, int N, int G, int dtype, int n_chunks, int chunk_rows,
-                              float* chunk_state, float* chunk_logdecay, void* stream) {
+                              float* chunk_state, float* chunk_logdecay, void* stream, int below_rows) {
   if (n_segments <= 0) return CBIS_OK;
+  if (below_rows > 0 && n_chunks != 1) return CBIS_ERR_BAD_SIZE;
   if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G) return CBIS_ERR_BAD_SIZE;
   if (n_chunks < 1 || (n_chunks > 1 && (chunk_rows < 1 || !chunk_state || !chunk_logdecay))) return CBIS_ERR_BAD_SIZE;
   if ((long long)n_segments * n_chunks > 65535 || H > 65535) return CBIS_ERR_TOO_LARGE;
@@ -446,11 +448,11 @@ CBIS_EXPORT int cbis_ssm_scan(const void* xbc, int xbc_ld, const void* proj, int
     if (dtype == CBIS_F32)
       return launch_scan<float>(xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, A_log, D, state, slot_stride, seg_slot,
                                 cu_rows, y, y_ld, n_segments, H, P, N, G, mode, n_chunks, chunk_rows, chunk_state,
-                                chunk_logdecay, st);
+                                chunk_logdecay, below_rows, st);
     if (dtype == CBIS_BF16)
       return launch_scan<__nv_bfloat16>(xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, A_log, D, state, slot_stride,
                                         seg_slot, cu_rows, y, y_ld, n_segments, H, P, N, G, mode, n_chunks, chunk_rows,
-                                        chunk_state, chunk_logdecay, st);
+                                        chunk_state, chunk_logdecay, below_rows, st);
     return CBIS_ERR_BAD_DTYPE;
   };
   if (n_chunks == 1) return run(0);

@@ -1,0 +1,59 @@
+"""The state-space recurrence 64 rows at a time, against the walk row by row in 64 bits."""
+import pytest
+import torch
+
+import plain_vekedra as pv
+
+pytestmark = pytest.mark.gpu
+
+
+def walk(xbc, raw, a_log, dt_bias, d_skip, H, P, N, G, S=None):
+    inner = H * P
+    x, B, C = xbc[:, :inner].view(-1, H, P), xbc[:, inner:inner + G * N].view(-1, G, N), xbc[:, inner + G * N:].view(-1, G, N)
+    B, C = (t.repeat_interleave(H // G, 1) for t in (B, C))
+    dt = pv.softplus(raw + dt_bias)
+    S = torch.zeros(H, P, N, dtype=torch.float64) if S is None else S
+    out = []
+    for t in range(x.shape[0]):
+        S = torch.exp(-torch.exp(a_log) * dt[t])[:, None, None] * S + dt[t][:, None, None] * x[t][:, :, None] * B[t][:, None, :]
+        out.append((S * C[t][:, None, :]).sum(-1) + d_skip[:, None] * x[t])
+    return torch.stack(out).view(-1, inner), S
+
+
+@pytest.mark.parametrize("H,P,N,G", [(2, 64, 128, 1), (4, 32, 64, 2), (3, 96, 64, 3)])
+def test_rows_in_chunks(H, P, N, G):
+    """Segments around a chunk's edges (33 rows and more go by chunks, fewer row by row, in one step), continued from their
+    states over several steps; one head that hardly decays, one whose decays underflow.  Each result is a sum of up to 700
+    32-bit terms around 1: bounded by 2e-6 of the largest, and no further off than the row-by-row kernel's."""
+    from cbis_b200.kernels import ops
+    g = torch.Generator().manual_seed(H * P)
+    inner = H * P
+    a_log, dt_bias, d_skip = torch.randn(H, generator=g), torch.randn(H, generator=g) - 1.0, torch.randn(H, generator=g)
+    a_log[0], dt_bias[0] = -5.0, -1.0
+    a_log[1] = 4.0
+    steps = [[64, 33, 1], [63, 200, 32], [129, 65, 700], [2, 34, 128]]
+    errs = {}
+    data = [[(torch.randn(n, inner + 2 * G * N, generator=g).bfloat16(), torch.randn(n, 3 + H, generator=g).bfloat16())
+             for n in s] for s in steps]
+    for how in (None, 0):      # by chunks; row by row
+        state = torch.zeros(4, inner * N + 5, dtype=torch.float32, device="cuda")
+        ref_S, worst = [None] * 3, 0.0
+        for sizes, seqs in zip(steps, data):
+            xs, ps = (torch.cat([s[i] for s in seqs]).cuda() for i in (0, 1))
+            cu = torch.tensor([0] + sizes, dtype=torch.int32).cumsum(0).int().cuda()
+            y = torch.full((sum(sizes), inner + 2), float("nan"), device="cuda")
+            ops.ssm_scan(xs, ps, 3, dt_bias.cuda(), a_log.cuda(), d_skip.cuda(), state, torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda"),
+                         cu, 3, H, P, N, G, y[:, :inner], max_seg_rows=max(sizes), piece_rows=how)
+            assert torch.isnan(y[:, inner:]).all()
+            at = 0
+            for i, n in enumerate(sizes):
+                ref, ref_S[i] = walk(seqs[i][0].double(), seqs[i][1][:, 3:].double(), a_log.double(), dt_bias.double(), d_skip.double(), H, P, N, G, ref_S[i])
+                worst = max(worst, ((y[at:at + n, :inner].double().cpu() - ref).abs().max() / ref.abs().max()).item())
+                at += n
+        for slot, i in ((2, 0), (0, 1), (1, 2)):
+            got = state[slot, :inner * N].view(H, P, N).double().cpu()
+            worst = max(worst, ((got - ref_S[i]).abs().max() / ref_S[i].abs().max()).item())
+        assert (state[3] == 0).all() and (state[:, inner * N:] == 0).all()
+        errs[how] = worst
+    print("largest relative error: chunks %.2e, row by row %.2e" % (errs[None], errs[0]))
+    assert errs[None] < 2e-6 and errs[None] <= errs[0], errs
