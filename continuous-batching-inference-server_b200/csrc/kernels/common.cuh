@@ -178,6 +178,27 @@ __device__ __forceinline__ float activate(float v, int act) {
   return v;
 }
 
+// The same for the N values a thread holds in registers: the choice is made once, not per value.  With the choice inside an
+// unrolled loop every value carried the code of all activations, tens of kilobytes that a warp jumps through: the epilogue
+// of the few-rows product at 64 rows spent 250 cycles a value on fetching instructions.
+template <int ACT, int N>
+__device__ __forceinline__ void activate_as(float (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = activate(v[i], ACT);
+}
+template <int N>
+__device__ __forceinline__ void activate_all(float (&v)[N], int act) {
+  switch (act) {
+    case CBIS_ACT_NONE: return;
+    case CBIS_ACT_GELU_ERF: return activate_as<CBIS_ACT_GELU_ERF>(v);
+    case CBIS_ACT_GELU_TANH: return activate_as<CBIS_ACT_GELU_TANH>(v);
+    case CBIS_ACT_SILU: return activate_as<CBIS_ACT_SILU>(v);
+    case CBIS_ACT_SIGMOID: return activate_as<CBIS_ACT_SIGMOID>(v);
+    case CBIS_ACT_RELU2: return activate_as<CBIS_ACT_RELU2>(v);
+    case CBIS_ACT_TANH: return activate_as<CBIS_ACT_TANH>(v);
+  }
+}
+
 // The inside of a gated feed-forward from the gate's and the up projection's sums.  limit > 0 cuts the gate off at
 // limit from above and the up value at -limit and limit; beta is silu's inner factor, g * sigmoid(beta g); shift is
 // added to the up value.  limit 0, beta 1, shift 0: act(g) * u.

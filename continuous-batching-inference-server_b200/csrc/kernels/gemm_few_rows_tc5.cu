@@ -222,8 +222,11 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     if (n < N) {
       const float b = bias ? bias[n] : 0.f;
 #pragma unroll
+      for (int m = 0; m < NT; ++m) v[m] += b;
+      activate_all(v, act);
+#pragma unroll
       for (int m = 0; m < NT; ++m)
-        if (m < M) from_f32(C[(size_t)m * ldc + n], activate(v[m] + b, act));
+        if (m < M) from_f32(C[(size_t)m * ldc + n], v[m]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -20,24 +20,32 @@ constexpr int TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 constexpr int TC_EPI_WARPS = 16;  // four per quarter of tensor memory, 64 columns each
 constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;  // warp 0: TMA, warp 1: MMA + tensor-memory allocation, then the epilogue
 
-// NC (16 or 32) consecutive columns of one row: bias, activation, ONE rounding, 16-byte stores where the row allows.
-template <typename TO, int NC = 32>
-__device__ __forceinline__ void store_row32(TO* dst, const float* v, const float* __restrict__ bias, int n, int N,
-                                            int act, bool vec_ok) {
-  float x[NC];
-  if (n + NC <= N) {
+// Adds the biases of NC columns from n on (of N): 16 bytes at a time where they allow it.
+template <int NC>
+__device__ __forceinline__ void add_bias(float (&x)[NC], const float* __restrict__ bias, int n, int N) {
+  if (bias == nullptr) return;
+  if (n + NC <= N && ((uintptr_t)(bias + n) & 15) == 0) {
 #pragma unroll
     for (int i = 0; i < NC; i += 4) {
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (bias) {
-        if (((uintptr_t)(bias + n) & 15) == 0) b = *reinterpret_cast<const float4*>(bias + n + i);
-        else b = make_float4(bias[n + i], bias[n + i + 1], bias[n + i + 2], bias[n + i + 3]);
-      }
-      x[i] = activate(v[i] + b.x, act);
-      x[i + 1] = activate(v[i + 1] + b.y, act);
-      x[i + 2] = activate(v[i + 2] + b.z, act);
-      x[i + 3] = activate(v[i + 3] + b.w, act);
+      const float4 b = __ldg(reinterpret_cast<const float4*>(bias + n + i));
+      x[i] += b.x;
+      x[i + 1] += b.y;
+      x[i + 2] += b.z;
+      x[i + 3] += b.w;
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) x[i] += n + i < N ? bias[n + i] : 0.f;
+  }
+}
+
+// NC (16 or 32) consecutive columns of one row: bias, activation, ONE rounding, 16-byte stores where the row allows.
+template <typename TO, int NC = 32>
+__device__ __forceinline__ void store_row32(TO* dst, float (&x)[NC], const float* __restrict__ bias, int n, int N,
+                                            int act, bool vec_ok) {
+  add_bias(x, bias, n, N);
+  activate_all(x, act);
+  if (n + NC <= N) {
     if (vec_ok) {
       if constexpr (sizeof(TO) == 2) {
 #pragma unroll
@@ -62,7 +70,9 @@ __device__ __forceinline__ void store_row32(TO* dst, const float* v, const float
     for (int i = 0; i < NC; ++i) from_f32(dst[i], x[i]);
     return;
   }
-  for (int i = 0; i < NC && n + i < N; ++i) from_f32(dst[i], activate(v[i] + (bias ? bias[n + i] : 0.f), act));
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (n + i < N) from_f32(dst[i], x[i]);
 }
 
 // Persistent: a block walks over tiles (tile, tile + gridDim.x, ...).  Two accumulators of 256 columns take
@@ -408,6 +418,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             if (n0 + c0 >= N) break;
             float v[32];
             tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + buf * TC_BN + (unsigned)c0, v);
+            add_bias(v, bias, n0 + c0, N);
+            activate_all(v, act);
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the store before has read `mine`
             __syncwarp();
 #pragma unroll
@@ -415,9 +427,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               unsigned pk[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                const int n = n0 + c0 + q * 8 + i * 2;
-                const float b0 = (bias && n < N) ? bias[n] : 0.f, b1 = (bias && n + 1 < N) ? bias[n + 1] : 0.f;
-                __nv_bfloat162 p = __floats2bfloat162_rn(activate(v[q * 8 + i * 2] + b0, act), activate(v[q * 8 + i * 2 + 1] + b1, act));
+                __nv_bfloat162 p = __floats2bfloat162_rn(v[q * 8 + i * 2], v[q * 8 + i * 2 + 1]);
                 pk[i] = *reinterpret_cast<unsigned*>(&p);
               }
               *reinterpret_cast<uint4*>(mine + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
@@ -444,18 +454,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             if (n0 + c0 >= N) break;
             float v[16];
             tmem_ld16(tmem_base + ((unsigned)(quarter * 32) << 16) + buf * TC_BN + (unsigned)c0, v);
+            add_bias(v, bias, n0 + c0, N);
+            activate_all(v, act);
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the copy before has read `mine`
             __syncwarp();
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float o[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int n = n0 + c0 + q * 4 + i;
-                o[i] = activate(v[q * 4 + i] + ((bias && n < N) ? bias[n] : 0.f), act);
-              }
-              *reinterpret_cast<float4*>(mine + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) = make_float4(o[0], o[1], o[2], o[3]);
-            }
+            for (int q = 0; q < 4; ++q)
+              *reinterpret_cast<float4*>(mine + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) =
+                  make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
