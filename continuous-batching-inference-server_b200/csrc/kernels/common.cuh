@@ -211,6 +211,59 @@ __device__ __forceinline__ float gated_product(float g, float u, int act, float 
   return a * (u + shift);
 }
 
+// The same for N pairs held in registers (the activation chosen once); the result replaces g.
+template <int N>
+__device__ __forceinline__ void gated_products(float (&g)[N], const float (&u)[N], int act, float limit, float beta, float shift) {
+  float up[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) up[i] = u[i];
+  if (limit > 0.f) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      g[i] = fminf(g[i], limit);
+      up[i] = fminf(fmaxf(up[i], -limit), limit);
+    }
+  }
+  if (act == CBIS_ACT_SILU) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) g[i] = g[i] * sigmoid_f32(beta * g[i]);
+  } else {
+    activate_all(g, act);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) g[i] *= up[i] + shift;
+}
+
+// Eight consecutive values, 16-byte aligned, as floats and back.
+__device__ __forceinline__ void load8(float (&v)[8], const float* p) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(float (&v)[8], const __nv_bfloat16* p) {
+  const uint4 r = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
+  uint4 r;
+  __nv_bfloat162 b0 = __floats2bfloat162_rn(v[0], v[1]), b1 = __floats2bfloat162_rn(v[2], v[3]);
+  __nv_bfloat162 b2 = __floats2bfloat162_rn(v[4], v[5]), b3 = __floats2bfloat162_rn(v[6], v[7]);
+  r.x = *reinterpret_cast<uint32_t*>(&b0);
+  r.y = *reinterpret_cast<uint32_t*>(&b1);
+  r.z = *reinterpret_cast<uint32_t*>(&b2);
+  r.w = *reinterpret_cast<uint32_t*>(&b3);
+  *reinterpret_cast<uint4*>(p) = r;
+}
+
 // What a head's distance bias takes off the score of a key `distance` positions back: slope * distance, or, for a head
 // with a rate, slope * ln(1 + rate * distance).
 __device__ __forceinline__ float distance_bias(float slope, const float* rate, float distance) {
