@@ -84,27 +84,41 @@ template <typename TT>
 __global__ void qk_prepare_kernel(TT* buf, int ld, int q_off, int q_heads, int k_off, int k_heads, int width,
                                   const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
                                   const int* positions, const float* __restrict__ freqs, int dims, int v_off, int d_v,
-                                  const TT* v_other, int v_other_ld, float lambda) {
+                                  const TT* v_other, int v_other_ld, float lambda, int table) {
+  // [q | k], then (table) the row's cosines and sines: every head turns by the same angles, which need nothing of the kernel before.
+  // (Taken anew for every head, and the two sums one after the other, a decode step's rows took 6.9 us.)
   extern __shared__ float row[];
-  __shared__ float red[33];
+  __shared__ float2 red[33];
   pdl_trigger();
-  pdl_wait();
   const int r = blockIdx.x;
   TT* b = buf + (size_t)r * ld;
-  const int d_q = q_heads * width, d_k = k_heads * width;
+  const int d_q = q_heads * width, d_k = k_heads * width, half = dims / 2;
+  float *cosines = row + d_q + d_k, *sines = cosines + half;
+  const float p = (float)positions[r];
+  if (table)
+    for (int i = threadIdx.x; i < half; i += blockDim.x) sincosf(p * freqs[i], &sines[i], &cosines[i]);
+  pdl_wait();
   float sq = 0.f, sk = 0.f;
+#pragma unroll 4
   for (int c = threadIdx.x; c < d_q + d_k; c += blockDim.x) {
     const float v = to_f32(c < d_q ? b[q_off + c] : b[k_off + c - d_q]);
     row[c] = v;
     if (c < d_q) sq += v * v;
     else sk += v * v;
   }
-  float inv_q = 1.f, inv_k = 1.f;
-  if (q_w) inv_q = 1.0f / sqrtf(block_sum(sq, red) / (float)d_q + eps);
-  if (k_w) inv_k = 1.0f / sqrtf(block_sum(sk, red) / (float)d_k + eps);
+  sq = warp_sum(sq);
+  sk = warp_sum(sk);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(sq, sk);
   __syncthreads();
-  const float p = (float)positions[r];
-  const int half = dims / 2, per_head = half + (width - dims);      // pairs, then entries that pass unrotated
+  if (threadIdx.x < 32) {
+    const float2 t = threadIdx.x < (blockDim.x + 31) >> 5 ? red[threadIdx.x] : make_float2(0.f, 0.f);
+    const float2 all = make_float2(warp_sum(t.x), warp_sum(t.y));
+    if (threadIdx.x == 0) red[32] = all;
+  }
+  __syncthreads();
+  const float inv_q = q_w ? 1.0f / sqrtf(red[32].x / (float)d_q + eps) : 1.f;
+  const float inv_k = k_w ? 1.0f / sqrtf(red[32].y / (float)d_k + eps) : 1.f;
+  const int per_head = half + (width - dims);      // pairs, then entries that pass unrotated
   for (int u = threadIdx.x; u < (q_heads + k_heads) * per_head; u += blockDim.x) {
     const int h = u / per_head, i = u % per_head;
     const bool is_q = h < q_heads;
@@ -120,7 +134,12 @@ __global__ void qk_prepare_kernel(TT* buf, int ld, int q_off, int q_heads, int k
         x1 *= w[c0 + i + half];
       }
       float sn, cs;
-      sincosf(p * freqs[i], &sn, &cs);
+      if (table) {
+        sn = sines[i];
+        cs = cosines[i];
+      } else {
+        sincosf(p * freqs[i], &sn, &cs);
+      }
       from_f32(dst[i], x0 * cs - x1 * sn);
       from_f32(dst[i + half], x1 * cs + x0 * sn);
     } else {
@@ -238,7 +257,9 @@ CBIS_EXPORT int cbis_qk_prepare(void* buf, int ld, int q_off, int q_heads, int k
     return CBIS_ERR_BAD_SIZE;
   const long long n = (long long)(q_heads + k_heads) * width;
   if (n > cbis_qk_prepare_max_width()) return CBIS_ERR_BAD_SIZE;
-  const size_t smem = (size_t)n * sizeof(float);
+  // the table of angles beside the row, unless both are more than a block can have
+  const int table = ((size_t)n + dims) * sizeof(float) <= 200 * 1024 ? 1 : 0;
+  const size_t smem = ((size_t)n + (table ? dims : 0)) * sizeof(float);
   const int threads = n >= 2048 ? 512 : (n >= 512 ? 256 : 128);
   cudaStream_t st = (cudaStream_t)stream;
 #define CBIS_QKP(TT)                                                                                                  \
@@ -247,7 +268,7 @@ CBIS_EXPORT int cbis_qk_prepare(void* buf, int ld, int q_off, int q_heads, int k
       cudaFuncSetAttribute(qk_prepare_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
     return (int)launch_pdl(qk_prepare_kernel<TT>, dim3(rows), dim3(threads), smem, st, (TT*)buf, ld, q_off, q_heads,  \
                            k_off, k_heads, width, q_w, k_w, eps, positions, freqs, dims, v_off, d_v,                  \
-                           (const TT*)v_other, v_other_ld, lambda);                                                   \
+                           (const TT*)v_other, v_other_ld, lambda, table);                                            \
   } while (0)
   if (dtype == CBIS_F32) CBIS_QKP(float);
   if (dtype == CBIS_BF16) CBIS_QKP(__nv_bfloat16);
