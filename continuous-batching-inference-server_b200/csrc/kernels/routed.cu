@@ -17,10 +17,10 @@ namespace cbis {
 
 constexpr int kScoreSigmoid = 0, kScoreSoftmax = 1;
 
-// grid (rows), 256 threads; shared: 2 (E + 1) floats.  ids [rows, top] int32, weights [rows, top] float.  correction (may
+// grid (rows), a warp for each router row up to 32; shared: 2 (E + 1) floats.  ids [rows, top] int32, weights [rows, top] float.  correction (may
 // be null): [E], added to the scores for the choice.  side (may be null): [rows], the sigmoid of router row E's logit.
 template <typename TT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 route_topk_kernel(const TT* h, int h_ld, const TT* __restrict__ router, int* ids, float* weights, int W, int E, int top,
                   int score, int renormalize, float renorm_eps, float weight_scale, const float* __restrict__ correction,
               float* side) {
@@ -32,7 +32,7 @@ route_topk_kernel(const TT* h, int h_ld, const TT* __restrict__ router, int* ids
   const TT* hr = h + (size_t)r * h_ld;
   constexpr int V = 16 / (int)sizeof(TT);      // elements of a 16-byte load
   const bool vec = W % V == 0 && !(((uintptr_t)hr | (uintptr_t)router) & 15);
-  for (int e = warp; e < E + (side ? 1 : 0); e += 8) {
+  for (int e = warp; e < E + (side ? 1 : 0); e += blockDim.x >> 5) {
     const TT* wr = router + (size_t)e * W;
     float acc = 0.f;
     if (vec) {
@@ -207,12 +207,16 @@ CBIS_EXPORT int cbis_route_topk(const void* h, int h_ld, const void* router, int
   if (E > 6000) return CBIS_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = (size_t)2 * (E + 1) * sizeof(float);
+  // few rows (decoding): a warp for every router row, so that no warp takes two rows of the router one after the other; many
+  // rows fill the SMs anyway, with eight warps each
+  const int warps = rows > 4 * 148 ? 8 : (E + 1 < 8 ? 8 : (E + 1 > 32 ? 32 : E + 1));
+  const dim3 block(32 * warps);
   if (dtype == CBIS_F32)
-    return (int)launch_pdl(route_topk_kernel<float>, dim3(rows), dim3(256), smem, st, (const float*)h, h_ld,
+    return (int)launch_pdl(route_topk_kernel<float>, dim3(rows), block, smem, st, (const float*)h, h_ld,
                            (const float*)router, ids, weights, W, E, top, score, renormalize, renorm_eps, weight_scale,
                            correction, side);
   if (dtype == CBIS_BF16)
-    return (int)launch_pdl(route_topk_kernel<__nv_bfloat16>, dim3(rows), dim3(256), smem, st, (const __nv_bfloat16*)h, h_ld,
+    return (int)launch_pdl(route_topk_kernel<__nv_bfloat16>, dim3(rows), block, smem, st, (const __nv_bfloat16*)h, h_ld,
                            (const __nv_bfloat16*)router, ids, weights, W, E, top, score, renormalize, renorm_eps,
                            weight_scale, correction, side);
   return CBIS_ERR_BAD_DTYPE;
