@@ -208,7 +208,8 @@ def _plain(ctx, mixer, qkv, cache, view, out, nd, T, hd, ps, k_pages, v_pages, k
                                             ctx.positions[d], out[d], mixer.n_head, mixer.n_kv_head, hd, ps, mixer.scale,
                                             mixer.window, chunks, partial)
             if ctx.n_segments > nd:
-                chunks, partial = _key_chunks(ctx, mixer.n_head, nd, T, hd)
+                # (three blocks fit on an SM; pieces for five times as many, so that the last ones leave few SMs idle)
+                chunks, partial = _key_chunks(ctx, mixer.n_head, nd, T, hd, blocks_per_sm=16)
                 ops.paged_prefill_f32(qkv, k_pages, v_pages, view.block_table, ctx.cu_rows, ctx.seg_start, out, nd,
                                       ctx.n_segments - nd, ctx.max_seg_rows, mixer.n_head, mixer.n_kv_head, hd, ps,
                                       mixer.scale, mixer.window, chunks, partial, ctx.positions, nd, T - nd)
