@@ -57,11 +57,20 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 // to cost the plain form a third of its speed: the two forms are separate kernels.)
 // GROUP: the output's columns come in groups with columns of A of their own.  TILES: row tiles of 16 over the blocks' second
 // index.  (Forms of their own: as run-time choices they cost a decode step of the others up to three per cent.)
-template <int MT, int NT, int UNROLL, bool LOW8, typename TO, bool CLUSTER = false, bool GROUP = false, bool TILES = false>
+// GLU: W holds the N gate rows and then the N up rows of a gated feed-forward; a block takes 8 of each, and the result is the
+// gated product of the two sums (`glu`).  The sums are rounded to bfloat16 first, as the product that writes them out
+// does: a token decoded alone and the same token in a prompt portion then meet the same roundings.
+struct GatedEpilogue {
+  float limit, beta, shift;
+  const float* row_gate;      // null, or a number per row that multiplies it
+};
+template <int MT, int NT, int UNROLL, bool LOW8, typename TO, bool CLUSTER = false, bool GROUP = false, bool TILES = false, bool GLU = false>
 __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int lda, const __nv_bfloat16* __restrict__ W,
                                                   const float* __restrict__ bias, TO* __restrict__ C, int ldc, int M,
                                                   int N, int K, int act, const void* next_w,
-                                                  unsigned long long next_bytes, int ksplit, int accumulate, int group_n, int act_from) {
+                                                  unsigned long long next_bytes, int ksplit, int accumulate, int group_n, int act_from,
+                                                  const GatedEpilogue* glu = nullptr) {
+  static_assert(!GLU || NT == 2, "a block of the gated form takes 8 gate and 8 up columns");
   extern __shared__ float red[];  // [SM_WARPS][MT*16][NT*8 + 1], then [ksplit - 1][MT*16 * NT*8] for the other blocks' sums
   constexpr int RS = NT * 8 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -70,7 +79,7 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
   int rank = 0;
   if constexpr (CLUSTER) rank = (int)cluster_ctarank();
   else ksplit = 1;
-  const int n0 = (blockIdx.x / ksplit) * (NT * 8);
+  const int n0 = (blockIdx.x / ksplit) * (GLU ? 8 : NT * 8);
   if constexpr (TILES) {
     const int m0 = blockIdx.y * 16;
     A += (size_t)m0 * lda;
@@ -95,7 +104,7 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
   const __nv_bfloat16* wrow[NT];
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
-    const int n = min(n0 + j * 8 + g, N - 1);  // rows past N are clamped; their columns are never stored
+    const int n = GLU ? min(n0 + g, N - 1) + j * N : min(n0 + j * 8 + g, N - 1);  // rows past N are clamped; their columns are never stored
     wrow[j] = W + (size_t)n * K + t * 8;
   }
   const __nv_bfloat16* arow[MT][2];
@@ -114,8 +123,14 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
   // starts it reads them from L2, and HBM keeps streaming while the short kernels in between run.
   if (threadIdx.x == 0) prefetch_share(next_w, next_bytes, blockIdx.x, gridDim.x);
   // the bias of this thread's first output column is fetched now (the epilogue maps idx -> column idx % (NT*8))
-  float bias0 = 0.f;
-  {
+  float bias0 = 0.f, bias1 = 0.f;
+  if constexpr (GLU) {
+    const int n = n0 + (int)(threadIdx.x & 7);
+    if (bias && n < N) {
+      bias0 = bias[n];
+      bias1 = bias[N + n];
+    }
+  } else {
     const int n = n0 + (int)(threadIdx.x % (NT * 8));
     if (bias && n < N) bias0 = bias[n];
   }
@@ -191,6 +206,25 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
    cluster_sync();
    if (rank > 0) return;
   }
+  if constexpr (GLU) {
+    for (int idx = threadIdx.x; idx < M * 8; idx += blockDim.x) {
+      const int m = idx >> 3, c = idx & 7, n = n0 + c;
+      if (n >= N) continue;
+      float v[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int w = 0; w < SM_WARPS; ++w) v[j] += red[((size_t)w * (MT * 16) + m) * RS + j * 8 + c];
+        if constexpr (CLUSTER)
+          for (int r = 1; r < ksplit; ++r) v[j] += others[(size_t)(r - 1) * (MT * 16) * (NT * 8) + m * (NT * 8) + j * 8 + c];
+      }
+      const float gate = to_f32(__float2bfloat16_rn(v[0] + bias0)), up = to_f32(__float2bfloat16_rn(v[1] + bias1));
+      float o = gated_product(gate, up, act, glu->limit, glu->beta, glu->shift);
+      if (glu->row_gate) o *= glu->row_gate[m];
+      from_f32(C[(size_t)m * ldc + n], o);
+    }
+    return;
+  }
   // blockDim (256) is a multiple of NT*8, so a thread meets the same column at every idx it takes
   for (int idx = threadIdx.x; idx < M * (NT * 8); idx += blockDim.x) {
     const int m = idx / (NT * 8), c = idx % (NT * 8);
@@ -230,6 +264,15 @@ gemm_small_m_low8_ksplit_kernel(const __nv_bfloat16* A, int lda, const __nv_bflo
                                 const float* __restrict__ bias, TO* __restrict__ C, int ldc, int M, int N, int K, int act,
                                 const void* next_w, unsigned long long next_bytes, int ksplit, int accumulate, int group_n, int act_from) {
   gemm_small_m_body<MT, NT, UNROLL, true, TO, true>(A, lda, W, bias, C, ldc, M, N, K, act, next_w, next_bytes, ksplit, accumulate, group_n, act_from);
+}
+
+// The gated form: up to 8 rows with K over the blocks of a cluster or not, and up to 16 rows.
+template <bool LOW8, bool CLUSTER>
+__global__ void __launch_bounds__(SM_WARPS * 32, LOW8 ? 4 : 3)
+gemm_small_m_gated_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
+                          __nv_bfloat16* __restrict__ C, int ldc, int M, int F, int K, int act, const void* next_w,
+                          unsigned long long next_bytes, int ksplit, const GatedEpilogue glu) {
+  gemm_small_m_body<1, 2, 4, LOW8, __nv_bfloat16, CLUSTER, false, false, true>(A, lda, W, bias, C, ldc, M, F, K, act, next_w, next_bytes, ksplit, 0, 0, 0, &glu);
 }
 
 template <int MT, int NT, int UNROLL, bool LOW8, typename TO, bool TILES = false>
@@ -336,4 +379,40 @@ CBIS_EXPORT int cbis_gemm_small_m_bf16(const void* A, int lda, const void* W, co
   if (out_dtype == CBIS_BF16) return dispatch_small_m<__nv_bfloat16>(A, lda, W, bias, C, ldc, M, N, K, act, next_w, next_bytes, st, 0, group_n, act_from);
   if (out_dtype == CBIS_F32) return dispatch_small_m<float>(A, lda, W, bias, C, ldc, M, N, K, act, next_w, next_bytes, st, accumulate, group_n, act_from);
   return CBIS_ERR_BAD_DTYPE;
+}
+
+// The inside of a gated feed-forward for up to 16 rows: C[M, F] = gated_product(A Wg^T + bg, A Wu^T + bu) (common.cuh) times
+// row_gate[m] where that is given; W [2 F, K] holds the gate rows, then the up rows, bias [2 F] or null alike.  C bfloat16.
+// One kernel instead of the product, which wrote both factors, and one that read them again.
+CBIS_EXPORT int cbis_gemm_small_m_gated_bf16(const void* A, int lda, const void* W, const float* bias, void* C, int ldc, int M,
+                                             int F, int K, int act, float limit, float beta, float shift, const float* row_gate,
+                                             const void* next_w, unsigned long long next_bytes, void* stream) {
+  if (M <= 0 || F <= 0) return CBIS_OK;
+  if (M > 16 || K <= 0 || K % 8 || lda < K || ldc < F) return CBIS_ERR_BAD_SIZE;
+  if (lda % 8 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)next_w & 15)) return CBIS_ERR_ALIGNMENT;
+  const GatedEpilogue glu = {limit, beta, shift, row_gate};
+  const int tiles = (F + 7) / 8, nkb = (K + 31) / 32;
+  int ks = 1;      // as dispatch_small_m splits K: few columns, one round of K blocks a warp
+  if (M <= 8 && ksplit_enabled())
+    while (ks < 4 && tiles * ks * 2 <= 4 * 148 && nkb >= SM_WARPS * 4 * ks * 2) ks *= 2;
+  const size_t smem = ((size_t)SM_WARPS * 16 * 17 + (size_t)(ks - 1) * 16 * 16) * sizeof(float);
+  // (more blocks than four an SM: the general form, three an SM, is the faster one, 11.5 us against 13.0 on 5,440 x 2,048)
+  auto kern = ks > 1 ? gemm_small_m_gated_kernel<true, true>
+                     : (M <= 8 && tiles > 3 * 148 && tiles <= 4 * 148 ? gemm_small_m_gated_kernel<true, false> : gemm_small_m_gated_kernel<false, false>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * ks));
+  cfg.blockDim = dim3(SM_WARPS * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)ks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ks > 1 ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)W, bias, (__nv_bfloat16*)C, ldc, M, F,
+                                 K, act, next_w, next_bytes, ks, glu);
 }

@@ -228,6 +228,29 @@ def gemm_small_m(x, w_nk, bias, act, out, accumulate=False, group_n: int = 0, ac
     _check(st, "gemm_small_m", f"M={M} N={N} K={K}")
 
 
+def gated_linear_takes(x, w_gate_up) -> bool:
+    """Whether ``gated_linear`` takes these rows: a few rows of bfloat16, aligned."""
+    return (x.dtype == torch.bfloat16 and x.shape[0] <= min(SMALL_M, 16) and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0)
+
+
+def gated_linear(x, w_gate_up, bias, act, out, row_gate=None, limit: float = 0.0, beta: float = 1.0, shift: float = 0.0):
+    """out = act(x @ Wg^T + bg) * (x @ Wu^T + bu) for up to 16 rows of bfloat16: the gated product of two products with the
+    rows of ``w_gate_up`` (the gate's, then the up projection's), whose sums are rounded to bfloat16 as ``linear`` does.  ``limit``,
+    ``beta``, ``shift``, ``row_gate``: as in ``gate_mul``."""
+    _need_cuda(x, w_gate_up, bias, out, row_gate)
+    M, K = x.shape
+    F = w_gate_up.shape[0] // 2
+    assert x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.is_contiguous() and w_gate_up.shape == (2 * F, K)
+    assert out.dtype == torch.bfloat16 and out.shape == (M, F) and x.stride(1) == 1 and out.stride(1) == 1
+    assert row_gate is None or (row_gate.dtype == torch.float32 and row_gate.numel() >= M and row_gate.is_contiguous())
+    nxt, nbytes = _next_of(w_gate_up)
+    st = kernels().cbis_gemm_small_m_gated_bf16(_ptr(x), c_int(x.stride(0)), _ptr(w_gate_up), _ptr(bias), _ptr(out),
+                                                c_int(out.stride(0)), c_int(M), c_int(F), c_int(K), c_int(ACT[act]), c_float(limit),
+                                                c_float(beta), c_float(shift), _ptr(row_gate), nxt, nbytes, _stream())
+    _check(st, "gated_linear", f"M={M} inner={F} K={K}")
+
+
 LN_LINEAR_MAX_ROWS = 8
 
 
@@ -1375,7 +1398,7 @@ def conv_state_update(x, c0, channels, taps, state, seg_slot, cu_rows, n_segment
 # measured on 2,048 rows (us, one piece -> pieces of 128 rows): 18 k state elements (segments x heads x columns x
 # states) 293 -> 81, 65 k 300 -> 147, 131 k 438 -> 252, 262 k 546 -> 476 or 473 -> 460, 524 k 578 -> 840: twice the
 # arithmetic pays only while one piece leaves most of the machine idle.
-SCAN_CHUNKS_FROM = 33           # rows of a segment from which it goes 64 rows at a time (a chunk of 33 rows costs what 12 rows of the walk do)
+SCAN_CHUNKS_FROM = 33           # rows of a segment from which it goes 64 rows at a time (a chunk takes 5 us, a row of the walk 0.28)
 SCAN_PIECE_ROWS = 128           # rows of a piece
 SCAN_PIECES_FROM = 384          # the longest segment of a step from which segments are cut
 SCAN_PIECES_MAX_STATE = 200_000  # state elements of a step up to which they are
