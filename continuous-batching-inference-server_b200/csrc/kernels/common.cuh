@@ -162,6 +162,16 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return red[32];
 }
 
+// The same for a block of 128 threads with one meeting instead of three: `red4` holds 4 floats, 16-byte aligned, used for
+// this sum alone.  (A decode step's norms are little else than their sums: 0.2 us a norm.)
+__device__ __forceinline__ float block_sum_128(float v, float* red4) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red4[threadIdx.x >> 5] = v;
+  __syncthreads();
+  const float4 t = *reinterpret_cast<const float4*>(red4);
+  return (t.x + t.y) + (t.z + t.w);
+}
+
 // Activations in 32-bit.  GELU, erf form: kernels/elementwise.cu:59-66 of the reference; tanh form: GPT-2's gelu_new;
 // silu(v) = v * sigmoid(v); sigmoid alone is the activation of a gate.
 __device__ __forceinline__ float sigmoid_f32(float v) { return 1.0f / (1.0f + expf(-v)); }

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(128)
 add_layernorm_reg_kernel(float* x, const TD* delta, const float* __restrict__ delta_bias,
                          const float* __restrict__ gamma, const float* __restrict__ beta, float eps, TO* __restrict__ out,
                          const int* rows, int d) {
-  __shared__ float red[33];
+  __shared__ __align__(16) float red[8];
   pdl_trigger();
   const int nvec = d >> 2;
   // parameters first: no earlier kernel writes them, so they are fetched while the kernels ahead still run
@@ -143,7 +143,7 @@ add_layernorm_reg_kernel(float* x, const TD* delta, const float* __restrict__ de
       sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     }
   }
-  const float mean = block_sum(sum, red) / (float)d;
+  const float mean = block_sum_128(sum, red) / (float)d;
   float sq = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -152,7 +152,7 @@ add_layernorm_reg_kernel(float* x, const TD* delta, const float* __restrict__ de
       sq += (a * a + b * b) + (c2 * c2 + e * e);
     }
   }
-  const float var = block_sum(sq, red) / (float)d;
+  const float var = block_sum_128(sq, red + 4) / (float)d;
   const float inv = rsqrtf(var + eps);
   const bool write_x = rows == nullptr && (drow != nullptr || delta_bias != nullptr);
   TO* orow = out + (size_t)r * d;

@@ -100,7 +100,7 @@ add_rmsnorm_reg_kernel(float* x, const TD* delta, int delta_ld, const float* __r
                        const float* __restrict__ post_w, float post_eps, float post_offset, const float* __restrict__ w,
                        float eps, float offset, TO* out, const int* rows, int d, float delta_scale, float x_scale,
                        const float* __restrict__ stream_w, float stream_eps, float stream_offset) {
-  __shared__ float red[33];
+  __shared__ __align__(16) float red[12];
   pdl_trigger();
   const int nvec = d >> 2;
   float4 wv[NV], pw[NV], db[NV];
@@ -137,7 +137,7 @@ add_rmsnorm_reg_kernel(float* x, const TD* delta, int delta_ld, const float* __r
     }
   }
   float dscale = 1.f;
-  if (drow && post_w) dscale = 1.0f / sqrtf(block_sum(ssd, red) / (float)d + post_eps);
+  if (drow && post_w) dscale = 1.0f / sqrtf(block_sum_128(ssd, red) / (float)d + post_eps);
   dscale *= delta_scale;
   float ss = 0.f;
 #pragma unroll
@@ -157,7 +157,7 @@ add_rmsnorm_reg_kernel(float* x, const TD* delta, int delta_ld, const float* __r
     }
   }
   if (stream_w) {
-    const float sinv = 1.0f / sqrtf(block_sum(ss, red) / (float)d + stream_eps);
+    const float sinv = 1.0f / sqrtf(block_sum_128(ss, red + 4) / (float)d + stream_eps);
     ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -170,7 +170,7 @@ add_rmsnorm_reg_kernel(float* x, const TD* delta, int delta_ld, const float* __r
       }
     }
   }
-  const float inv = w ? 1.0f / sqrtf(block_sum(ss, red) / (float)d + eps) : 1.f;      // no weight: the rows go on as they are
+  const float inv = w ? 1.0f / sqrtf(block_sum_128(ss, red + 8) / (float)d + eps) : 1.f;      // no weight: the rows go on as they are
   const bool write_x = rows == nullptr && (drow != nullptr || stream_w != nullptr || x_scale != 1.f);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
