@@ -118,6 +118,7 @@ class ModelRunner:
         self.feed_tokens = None   # int32 tokens on the device that replace the next packed step's (single-token entries, in order)
         self.last_info = None
         self._stream_obj = None
+        self._branch = None
         # decode-only steps replay a captured CUDA graph unless a part reads device values on the host
         self.use_graphs = all(getattr(part, "capturable", True) for _, part in model.all_parts())
         self._graphs: Dict[tuple, tuple] = {}    # (rows of a decode-only step, context class) -> (graph, logits)
@@ -160,6 +161,15 @@ class ModelRunner:
         self._scratch = torch.empty(max(worst, 1), dtype=torch.float32, device=self.device)
         self._counters = torch.zeros(max(S * heads, 1), dtype=torch.int32, device=self.device)
         self.graph_replays = 0
+
+    def branch_stream(self):
+        """A second stream for independent kernels of a step that is being captured (they become branches of the graph);
+        None in a step that runs launch by launch: there the host, which pays for the events, is what is short."""
+        if not torch.cuda.is_current_stream_capturing():
+            return None
+        if self._branch is None:
+            self._branch = torch.cuda.Stream()
+        return self._branch
 
     # ------------------------------------------------------------------
     def _dev_view(self, name, n=None):
