@@ -369,7 +369,7 @@ class Engine:
                 n = min(self.runner.max_tokens, len(tokens) - pos)
                 outs.append(self.forward_step([StepEntry(slot, pos, list(tokens[pos:pos + n]), list(range(n)))]))
                 pos += n
-            return torch.cat(outs)
+            return outs[0].contiguous() if len(outs) == 1 else torch.cat(outs)      # one portion's rows are the caller's already
         finally:
             self.close_request(slot)
 
