@@ -172,6 +172,19 @@ __device__ __forceinline__ float block_sum_128(float v, float* red4) {
   return (t.x + t.y) + (t.z + t.w);
 }
 
+// Bytes of dynamic shared memory to launch a kernel of `blocks` blocks with, so that no more of them fit on an SM than an even
+// spread over the 148 puts there: `need`, or more.  Blocks that start while the kernel ahead still runs are packed onto the SMs it
+// leaves idle, as many as fit, and those SMs then take as much longer (a 32-bit product of 512 x 256 x 1024, 128 blocks: 20 us
+// alone, 51 in a chain; 20 in either so).  Sets the kernel's limit to one value whatever the size: another thread may be between
+// its call of this and its launch.
+template <typename Kern>
+inline cudaError_t spread_evenly(Kern kern, long long blocks, size_t need, size_t* smem) {
+  const long long per_sm = (blocks + 147) / 148;
+  const size_t share = 227 * 1024 / (size_t)(per_sm + 1);      // one block more would not fit
+  *smem = share > need ? share : need;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+}
+
 // Activations in 32-bit.  GELU, erf form: kernels/elementwise.cu:59-66 of the reference; tanh form: GPT-2's gelu_new;
 // silu(v) = v * sigmoid(v); sigmoid alone is the activation of a gate.
 __device__ __forceinline__ float sigmoid_f32(float v) { return 1.0f / (1.0f + expf(-v)); }

@@ -77,7 +77,7 @@ linear_f32_kernel(const float* A, const float* __restrict__ W, const float* __re
 // More than 16 rows with W stored [N, K] (both operands contiguous along k, 16-byte aligned): tiles of BM x BN
 // outputs, k in pieces of 32 that arrive by 16-byte cp.async in a ring of buffers (the next pieces are on their way while
 // this one is multiplied), operands kept [row][k] in shared memory so that the copy is straight and a thread reads
-// four k of a row at once.  A thread owns the outputs (ty + 16 i, tx + 16 j) and walks k from left to right with
+// four k of a row at once.  A thread owns TM x TN outputs, TY rows and TX columns apart, and walks k from left to right with
 // one fused multiply-add per element: the order of the kernels above and below, hence the same bits.  The tile
 // shrinks (64x64, 32x64, 32x32) until the grid fills the SMs: a 512 x 256 x 1024 product had 8 blocks of the
 // 128 x 128 kernel above and took 190 us.
@@ -93,28 +93,31 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // NK_STAGES pieces are in the ring: a piece of a 32 x 32 tile is multiplied in 0.3 us, a trip to L2 takes 0.7, so with two
-// buffers a block waited most of its time (the two products of 512 rows with 256 columns, K 256 and 1,024: 55 us on average, now 29).
+// buffers a block waited most of its time (the two products of 512 rows with 256 columns, K 256 and 1,024: 55 us on average; 29 with the ring, 14 with the blocks spread evenly as well).
 constexpr int NK_STAGES = 5;
-template <int BM, int BN>
-__global__ void __launch_bounds__(256)
+// A thread owns TM x TN outputs: with more a load from shared memory serves more multiply-adds, with fewer a block has the
+// warps to hide a load's trip.  32 x 64: 4 x 4 (512 x 768 x 256: 14.8 us, 2 x 4: 15.9); 32 x 32, a grid that gives an SM one block:
+// 2 x 2 (512 x 256 x 1024: 20 us, 2 x 4: 28, 4 x 4: 39).
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
 linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                      int M, int N, int K, int act, int lda, int ldc) {
-  constexpr int BK = 32, PITCH = BK + 4, TM = BM / 16, TN = BN / 16;
+  constexpr int BK = 32, PITCH = BK + 4, TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
   extern __shared__ __align__(16) float nk_smem[];
   float (*As)[BM][PITCH] = reinterpret_cast<float (*)[BM][PITCH]>(nk_smem);                              // [NK_STAGES][BM][PITCH]
   float (*Ws)[BN][PITCH] = reinterpret_cast<float (*)[BN][PITCH]>(nk_smem + NK_STAGES * BM * PITCH);     // [NK_STAGES][BN][PITCH]
   pdl_trigger();
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   auto load_w = [&](int k0, int stage) {
-    for (int i = tid; i < BN * (BK / 4); i += 256) {
+    for (int i = tid; i < BN * (BK / 4); i += THREADS) {
       const int r = i / (BK / 4), c = (i % (BK / 4)) * 4;
       const bool valid = n0 + r < N && k0 + c < K;
       cp_async16_f32(&Ws[stage][r][c], valid ? W + (size_t)(n0 + r) * K + k0 + c : W, valid);
     }
   };
   auto load_a = [&](int k0, int stage) {
-    for (int i = tid; i < BM * (BK / 4); i += 256) {
+    for (int i = tid; i < BM * (BK / 4); i += THREADS) {
       const int r = i / (BK / 4), c = (i % (BK / 4)) * 4;
       const bool valid = m0 + r < M && k0 + c < K;
       cp_async16_f32(&As[stage][r][c], valid ? A + (size_t)(m0 + r) * lda + k0 + c : A, valid);
@@ -143,13 +146,12 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
     }
     cp_async_commit();
     const int kc = min(BK, K - kt * BK);   // a multiple of 4; the sum stops at K (0 * 0 could still flip the sign of a zero)
-#pragma unroll 2
-    for (int kk = 0; kk < kc; kk += 4) {
+    auto four = [&](int kk) {
       float4 a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(&As[stage][ty + 16 * i][kk]);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(&As[stage][ty + TY * i][kk]);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(&Ws[stage][tx + 16 * j][kk]);
+      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(&Ws[stage][tx + TX * j][kk]);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -161,15 +163,21 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
           v = fmaf(a[i].w, b[j].w, v);
           acc[i][j] = v;
         }
+    };
+    if (kc == BK) {
+#pragma unroll
+      for (int kk = 0; kk < BK; kk += 4) four(kk);
+    } else {
+      for (int kk = 0; kk < kc; kk += 4) four(kk);
     }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty + 16 * i;
+    const int m = m0 + ty + TY * i;
     if (m >= M) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx + 16 * j;
+      const int n = n0 + tx + TX * j;
       if (n >= N) continue;
       float v = acc[i][j];
       if (bias) v += bias[n];
@@ -187,7 +195,7 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 // alone and the same token inside a prompt portion still agree exactly.
 // With 16-byte aligned rows (linear_f32_few_rows_kernel<true>) up to four pieces are on their way at once, the weights' since
 // before the wait for the kernel ahead: piece by piece, each a trip to L2 with nothing else to do, the products of a
-// 256-wide model's decode step took 6.7 us on average; now 4.9.
+// 256-wide model's decode step took 6.7 us on average; 5.2 so, 4.8 with the blocks spread evenly (common.cuh).
 constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4, FR_STAGES = 4;
 __device__ __forceinline__ float few_rows_walk(const float* a, const float* w, int kc, float acc) {
   int k = 0;
@@ -284,20 +292,18 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
     // (a 128 x 128 tile, 8 x 8 outputs a thread, was measured too: 198 registers, one block per SM, no faster than 64 x 64)
     const long long b64 = (long long)((M + 63) / 64) * ((N + 63) / 64),
                     b32 = (long long)((M + 31) / 32) * ((N + 63) / 64);
-#define CBIS_NK(BM_, BN_)                                                                                              \
+#define CBIS_NK(BM_, BN_, TM_, TN_)                                                                                    \
   {                                                                                                                    \
-    auto kern = linear_f32_nk_kernel<BM_, BN_>;                                                                        \
-    const size_t smem = (size_t)NK_STAGES * (BM_ + BN_) * 36 * sizeof(float);                                                  \
-    if (smem > 48 * 1024) {                                                                                            \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
-      if (e != cudaSuccess) return (int)e;                                                                             \
-    }                                                                                                                  \
-    return (int)launch_pdl(kern, dim3((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_), dim3(256), smem, st, A, W, bias, C, M, N, K, \
-                           act, lda, ldc);                                                                             \
+    auto kern = linear_f32_nk_kernel<BM_, BN_, TM_, TN_>;                                                              \
+    const dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);                                                         \
+    size_t smem;                                                                                                       \
+    cudaError_t e = spread_evenly(kern, (long long)grid.x * grid.y, NK_STAGES * (BM_ + BN_) * 36 * sizeof(float), &smem); \
+    if (e != cudaSuccess) return (int)e;                                                                               \
+    return (int)launch_pdl(kern, grid, dim3((BM_ / TM_) * (BN_ / TN_)), smem, st, A, W, bias, C, M, N, K, act, lda, ldc); \
   }
-    if (b64 >= 2 * 148) CBIS_NK(64, 64)
-    if (b32 >= 148) CBIS_NK(32, 64)
-    CBIS_NK(32, 32)
+    if (b64 >= 2 * 148) CBIS_NK(64, 64, 4, 4)
+    if (b32 >= 148) CBIS_NK(32, 64, 4, 4)
+    CBIS_NK(32, 32, 2, 2)
 #undef CBIS_NK
   }
   if (M > 256) {
@@ -314,11 +320,9 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
     auto kern = aligned ? linear_f32_few_rows_kernel<true> : linear_f32_few_rows_kernel<false>;
     const int pieces = (K + FR_KC - 1) / FR_KC, stages = !aligned ? 1 : (pieces < FR_STAGES ? pieces : FR_STAGES);
-    const size_t smem = (size_t)stages * 32 * FR_PITCH * sizeof(float);
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return (int)e;
-    }
+    size_t smem;
+    cudaError_t e = spread_evenly(kern, (N + 15) / 16, (size_t)stages * 32 * FR_PITCH * sizeof(float), &smem);
+    if (e != cudaSuccess) return (int)e;
     return (int)launch_pdl(kern, dim3((N + 15) / 16), dim3(256), smem, st, A, W, bias, C, M, N, K, act, lda, ldc);
   }
   dim3 grid((N + 63) / 64, (M + 15) / 16);
