@@ -133,7 +133,9 @@ class ModelRunner:
         # ... and, whatever a step costs the host, once its launches have cost as much as a capture does: a step of the
         # reference's sizes (0.7 ms of launches around 0.25 ms of kernels) after some ninety times
         self.shape_graph_capture_s = 60e-3
-        self._shape_seen: Dict[tuple, int] = {}
+        # shape -> [times seen, host seconds of its last launch-by-launch run, step it is counted from, step it last came in]
+        self._shape_seen: Dict[tuple, list] = {}
+        self._shape_steps = 0
         self._shape_graphs: "OrderedDict[tuple, tuple]" = OrderedDict()
         self.shape_captures = self.shape_replays = 0
         # Small steps with prompt portions (up to small_step_rows rows) whose launches cost the host more than the
@@ -435,6 +437,12 @@ class ModelRunner:
         milliseconds: for a small model that is a hundred steps, and its steps cost the host little anyway), or
         returns None (the caller then runs the step launch by launch).  A cheaper shape is captured once its launches have
         cost the host what the capture will."""
+        self._shape_steps += 1
+        if len(self._shape_seen) > 4096:      # the shapes with a graph keep their counts
+            self._shape_seen = {s: r for s, r in self._shape_seen.items() if s in self._shape_graphs}
+        seen = self._shape_seen.setdefault(shape, [0, 0.0, self._shape_steps, 0])
+        seen[0] += 1
+        seen[3] = self._shape_steps
         have = self._shape_graphs.get(shape)
         if have is not None:
             self._shape_graphs.move_to_end(shape)
@@ -444,12 +452,10 @@ class ModelRunner:
             self.graph_replays += 1
             self.shape_replays += 1
             return logits
-        if len(self._shape_seen) > 4096:
-            self._shape_seen.clear()
-        seen = self._shape_seen.setdefault(shape, [0, 0.0])      # [times seen, host seconds of the last launch-by-launch run]
-        seen[0] += 1
         if seen[0] < self.shape_graph_after or (seen[1] < self.shape_graph_min_host_s
                                                 and seen[0] * seen[1] < self.shape_graph_capture_s):
+            return None
+        if len(self._shape_graphs) >= self.max_shape_graphs and not self._takes_a_place(seen):
             return None
         ctx = self.build_context(entries, fixed_shapes=True)
         # The step itself runs ONCE, launch by launch, with the launches the graph will hold; the capture that
@@ -459,11 +465,25 @@ class ModelRunner:
         first = self.model.forward(ctx)
         graph, logits = capture_graph(lambda: self.model.forward(ctx))
         logits.copy_(first)
-        while len(self._shape_graphs) >= self.max_shape_graphs:
-            self._shape_graphs.popitem(last=False)        # the shape not used for the longest time makes room
+        while len(self._shape_graphs) >= self.max_shape_graphs:      # its shape is counted anew from here on
+            del self._shape_seen[self._shape_graphs.popitem(last=False)[0]]
         self._shape_graphs[shape] = (graph, logits)
         self.shape_captures += 1
         return logits
+
+    def _takes_a_place(self, seen: list) -> bool:
+        """With a graph in every place: whether the shape counted in ``seen`` takes the place of the one whose graph was
+        not used for the longest time.  It does if that one did not come at all while the newcomer was counted, or comes
+        less than half as often.  Otherwise the newcomer's count begins anew and the other's history loses half its
+        weight.  (Were the last one to come given the place at once, one shape more than there are places, in rotation,
+        would make every step a capture: 60 ms instead of 0.7.)"""
+        now, old = self._shape_steps, self._shape_seen[next(iter(self._shape_graphs))]
+        age, since = now - old[2] + 1, now - seen[2] + 1
+        if old[3] < seen[2] or seen[0] * age > 2 * old[0] * since:
+            return True
+        seen[0], seen[2] = 0, now + 1
+        old[0], old[2] = old[0] / 2, now - age // 2
+        return False
 
     def _decode_step_graph(self, entries, native: bool) -> torch.Tensor:
         rows = self._bucket(len(entries))
