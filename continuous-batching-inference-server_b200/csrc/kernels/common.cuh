@@ -163,13 +163,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // The same for a block of 128 threads with one meeting instead of three: `red4` holds 4 floats, 16-byte aligned, used for
-// this sum alone.  (A decode step's norms are little else than their sums: 0.2 us a norm.)
+// this sum alone.  (A decode step's norms are little else than their sums: 0.2 us a norm.)  The warps' sums are added in the order
+// in which block_sum's shuffles add them, so that a row's norm has the same bits whichever of the two its kernel uses.
 __device__ __forceinline__ float block_sum_128(float v, float* red4) {
   v = warp_sum(v);
   if ((threadIdx.x & 31) == 0) red4[threadIdx.x >> 5] = v;
   __syncthreads();
   const float4 t = *reinterpret_cast<const float4*>(red4);
-  return (t.x + t.y) + (t.z + t.w);
+  return (t.x + t.z) + (t.y + t.w);
 }
 
 // Bytes of dynamic shared memory to launch a kernel of `blocks` blocks with, so that no more of them fit on an SM than an even
