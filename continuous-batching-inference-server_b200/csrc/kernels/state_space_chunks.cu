@@ -51,15 +51,34 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two neighbouring values into three bfloat16 parts each, `part` elements apart.
+// Two neighbouring values into three bfloat16 parts each, `part` elements apart.  An infinite value (or none) is its first part
+// alone: infinity less infinity would be no number; a value that only rounds to infinity has the largest bfloat16 as its first.
 __device__ __forceinline__ void store_parts(__nv_bfloat16* at, int part, float v0, float v1) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
-    *reinterpret_cast<__nv_bfloat162*>(at + i * part) = b;
-    v0 -= __low2float(b);
-    v1 -= __high2float(b);
+  __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
+  float r0 = v0 - __low2float(b), r1 = v1 - __high2float(b);
+  const uint32_t bits = *reinterpret_cast<const uint32_t*>(&b);
+  if ((bits & 0x7F80u) == 0x7F80u || (bits & 0x7F800000u) == 0x7F800000u) {
+    constexpr float TOP = 3.3895313892515355e38f;
+    const bool f0 = fabsf(v0) < INFINITY, f1 = fabsf(v1) < INFINITY;
+    b = __floats2bfloat162_rn(f0 ? fminf(fmaxf(v0, -TOP), TOP) : v0, f1 ? fminf(fmaxf(v1, -TOP), TOP) : v1);
+    r0 = f0 ? v0 - __low2float(b) : 0.f;
+    r1 = f1 ? v1 - __high2float(b) : 0.f;
   }
+  *reinterpret_cast<__nv_bfloat162*>(at) = b;
+#pragma unroll
+  for (int i = 1; i < 3; ++i) {
+    b = __floats2bfloat162_rn(r0, r1);
+    *reinterpret_cast<__nv_bfloat162*>(at + i * part) = b;
+    r0 -= __low2float(b);
+    r1 -= __high2float(b);
+  }
+}
+// Whether one of the eight bfloat16 of a fragment is infinite or no number.
+__device__ __forceinline__ bool not_finite(const uint32_t (&r)[4]) {
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) bad |= (r[i] & 0x7F80u) == 0x7F80u || (r[i] & 0x7F800000u) == 0x7F800000u;
+  return bad;
 }
 
 template <int N>
@@ -236,6 +255,20 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
     for (int k = 0; k <= t0; k += 16) {
       uint32_t a[4], b[4];
       ldm_t(b, sX + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + py + (lane >> 4) * 8);
+      if (k == t0 && __any_sync(0xffffffffu, not_finite(b))) {
+        // the zeros above the diagonal times an infinite x of a later row would be no number: these rows one by one, to their own
+        for (int s1 = 0; s1 < 16; ++s1)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int r1 = g + 8 * (e >> 1);
+            if (s1 > r1) continue;
+            const __nv_bfloat16* m = sm + T::M0 + (t0 + r1) * MP + t0 + s1;
+            const float w = to_f32(m[0]) + (to_f32(m[Q * MP]) + to_f32(m[2 * Q * MP]));
+#pragma unroll
+            for (int j = 0; j < 2; ++j) first[j][e] = fmaf(w, to_f32(sX[(t0 + s1) * XP + py + 8 * j + 2 * t4 + (e & 1)]), first[j][e]);
+          }
+        break;
+      }
 #pragma unroll
       for (int part = 0; part < 3; ++part) {
         ldm(a, sm + T::M0 + part * Q * MP + (t0 + (lane & 15)) * MP + k + (lane >> 4) * 8);

@@ -57,3 +57,26 @@ def test_rows_in_chunks(H, P, N, G):
         errs[how] = worst
     print("largest relative error: chunks %.2e, row by row %.2e" % (errs[None], errs[0]))
     assert errs[None] < 2e-6 and errs[None] <= errs[0], errs
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), -float("inf")])
+@pytest.mark.parametrize("at", [0, 37, 47, 70])
+def test_an_infinite_x_reaches_its_own_column_from_its_own_row_on(value, at):
+    """One x that is no finite number, at a tile's edge or inside it: the rows before it and all other columns, of y and of the
+    state, are what they are with a 0 in its place (the bound of the test above), its column is not finite from there on."""
+    from cbis_b200.kernels import ops
+    H, P, N, rows, col = 2, 64, 128, 100, 21
+    g = torch.Generator().manual_seed(at)
+    xbc, raw = torch.randn(rows, H * P + 2 * N, generator=g).bfloat16(), torch.randn(rows, H, generator=g).bfloat16()
+    a_log, dt_bias, d_skip = torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda()
+    out = []
+    for v in (0.0, value):
+        xbc[at, col] = v
+        state, y = torch.zeros(1, H * P * N, device="cuda"), torch.empty(rows, H * P, device="cuda")
+        ops.ssm_scan(xbc.cuda(), raw.cuda(), 0, dt_bias, a_log, d_skip, state, torch.zeros(1, dtype=torch.int32, device="cuda"),
+                     torch.tensor([0, rows], dtype=torch.int32, device="cuda"), 1, H, P, N, 1, y, max_seg_rows=rows)
+        out.append((y.cpu(), state.view(H * P, N).cpu()))
+    (y0, s0), (y1, s1) = out
+    assert not torch.isfinite(y1[at:, col]).any() and not torch.isfinite(s1[col]).any()
+    y1[at:, col], s1[col] = y0[at:, col], s0[col]
+    assert (y1 - y0).abs().max() <= 2e-6 * y0.abs().max() and (s1 - s0).abs().max() <= 2e-6 * s0.abs().max()
