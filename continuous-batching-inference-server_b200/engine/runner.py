@@ -169,8 +169,8 @@ class ModelRunner:
         None in a step that runs launch by launch: there the host, which pays for the events, is what is short."""
         if not torch.cuda.is_current_stream_capturing():
             return None
-        if self._branch is None:
-            self._branch = torch.cuda.Stream()
+        if self._branch is None:      # no other holder: nobody else's launches get into the capture
+            self._branch = ops.own_stream(self, self.device)
         return self._branch
 
     # ------------------------------------------------------------------

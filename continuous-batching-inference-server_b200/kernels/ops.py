@@ -82,6 +82,16 @@ def raw_stream_handle():
     return None
 
 
+def own_stream(owner, device) -> torch.cuda.ExternalStream:
+    """A stream that only ``owner`` holds, for as long as ``owner`` lives.  (``torch.cuda.Stream()`` hands out 32 streams in
+    turn: another holder may have the same one.)"""
+    handle, lib = c_void_p(), kernels()
+    with torch.cuda.device(device):
+        _check(lib.cbis_stream_create(ctypes.byref(handle)), "stream_create", launches=0)
+    weakref.finalize(owner, lib.cbis_stream_destroy, c_void_p(handle.value)).atexit = False
+    return torch.cuda.ExternalStream(handle.value, device=device)
+
+
 def _need_cuda(*ts):
     for t in ts:
         if t is not None and not t.is_cuda:
