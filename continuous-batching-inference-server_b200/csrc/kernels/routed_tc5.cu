@@ -16,6 +16,7 @@
 //
 // Every wait on an mbarrier is bounded: when one runs out the block sets *error, waits for its copies and products in
 // flight, frees its tensor memory and returns.
+#include "routed_mma.cuh"
 #include "tc5_common.cuh"
 
 namespace cbis {
@@ -288,7 +289,11 @@ template <bool DUAL>
 static int launch(const void* a, int places, int K, const void* b, long long b_total, int b_rows, int N, const int* sorted,
                   const float* weights, const int* tile_expert, const int* tile_start, const int* tile_rows, const int* n_tiles,
                   int max_tiles, void* out, int act, int weight_on_input, float limit, float beta, float shift, int* error,
-                  cudaStream_t st) {
+                  int tc5, cudaStream_t st) {
+  if (!tc5)
+    return (int)launch_pdl(routed_mma_kernel<DUAL>, dim3(max_tiles, (N + MM_N - 1) / MM_N), dim3(256), 0, st, (const __nv_bfloat16*)a,
+                           (const __nv_bfloat16*)b, sorted, weights, tile_expert, tile_start, tile_rows, n_tiles, out, N, K, b_rows,
+                           act, weight_on_input, limit, beta, shift);
   CUtensorMap map_a, map_b;
   int s = make_map(&map_a, a, places, K, K, TILE_M);
   if (s == CBIS_OK) s = make_map(&map_b, b, (int)b_total, K, K, TILE_N / 2);
@@ -318,18 +323,19 @@ CBIS_EXPORT long long cbis_routed_plan_ints(int pairs, int E) {
 
 // The whole routed feed-forward for many rows of bfloat16.  plan: cbis_routed_plan_ints ints; x [pairs, W] and hid
 // [pairs, F] bfloat16; y [pairs, W] 32-bit; out [rows, W] 32-bit, overwritten, or added to with `accumulate`.  W and F are
-// multiples of 8.  error: int on the device, set non-zero if a wait inside a kernel ran out.
+// multiples of 8.  tc5: the products on TMA + tcgen05 (or on mma.sync, which matrices with more rows than a coordinate counts take
+// in any case); error: int on the device, set non-zero if a wait inside those kernels ran out.
 CBIS_EXPORT int cbis_routed_tiles(const void* h, int h_ld, const void* gate_up, const void* down, const int* ids,
                                   const float* weights, int* plan, void* x, void* hid, float* y, float* out, int out_ld, int rows,
                                   int W, int F, int E, int top, int act, int weight_on_input, int accumulate,
-                                  void* stream, float limit, float beta, float shift, int* error) {
+                                  void* stream, float limit, float beta, float shift, int* error, int tc5) {
   if (rows <= 0) return CBIS_OK;
   if (W <= 0 || F <= 0 || E <= 0 || top <= 0) return CBIS_ERR_BAD_SIZE;
   if (W % 8 || F % 8 || h_ld % 8) return CBIS_ERR_ALIGNMENT;
   if (((uintptr_t)h | (uintptr_t)gate_up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)hid | (uintptr_t)y) & 15) return CBIS_ERR_ALIGNMENT;
-  if (error == nullptr) return CBIS_ERR_ALIGNMENT;
-  if (E > 4096 || (long long)rows * top > 0x3fffffffLL || 2ll * E * F > 0x7fffffffLL || (long long)E * W > 0x7fffffffLL)
-    return CBIS_ERR_TOO_LARGE;
+  if (E > 4096 || (long long)rows * top > 0x3fffffffLL) return CBIS_ERR_TOO_LARGE;
+  tc5 = tc5 && 2ll * E * F <= 0x7fffffffLL && (long long)E * W <= 0x7fffffffLL;
+  if (tc5 && error == nullptr) return CBIS_ERR_ALIGNMENT;
   cudaStream_t st = (cudaStream_t)stream;
   const int pairs = rows * top;
   const int max_tiles = (pairs + rt::TILE_M - 1) / rt::TILE_M + E;
@@ -347,10 +353,10 @@ CBIS_EXPORT int cbis_routed_tiles(const void* h, int h_ld, const void* gate_up, 
                    (const int*)sorted, (__nv_bfloat16*)x, W, E, top);
   if (err != cudaSuccess) return (int)err;
   int s = rt::launch<true>(x, pairs, W, gate_up, 2ll * E * F, 2 * F, F, sorted, weights, tile_expert, tile_start, tile_rows,
-                           n_tiles, max_tiles, hid, act, weight_on_input, limit, beta, shift, error, st);
+                           n_tiles, max_tiles, hid, act, weight_on_input, limit, beta, shift, error, tc5, st);
   if (s != CBIS_OK) return s;
   s = rt::launch<false>(hid, pairs, F, down, (long long)E * W, W, W, sorted, weights, tile_expert, tile_start, tile_rows,
-                        n_tiles, max_tiles, y, act, weight_on_input, limit, beta, shift, error, st);
+                        n_tiles, max_tiles, y, act, weight_on_input, limit, beta, shift, error, tc5, st);
   if (s != CBIS_OK) return s;
   return (int)launch_pdl(rt::routed_combine_kernel, dim3(rows), dim3(256), 0, st, (const float*)y, (const int*)place, out, out_ld, W,
                          top, accumulate, ids, weights, E, (const __nv_bfloat16*)h, h_ld);

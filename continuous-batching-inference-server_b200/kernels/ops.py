@@ -1528,7 +1528,7 @@ ROUTED_TILES_FROM = 33     # rows from which the routed feed-forward sorts its r
 def routed_tiles_takes(h, gate_up, down) -> bool:
     """Whether ``routed_tiles`` takes these rows: bfloat16, enough of them, sizes in steps of 8, aligned."""
     W, F = gate_up.shape[2], down.shape[2]
-    return (USE_TCGEN05 and h.dtype == torch.bfloat16 and h.shape[0] >= ROUTED_TILES_FROM and W % 8 == 0 and F % 8 == 0
+    return (h.dtype == torch.bfloat16 and h.shape[0] >= ROUTED_TILES_FROM and W % 8 == 0 and F % 8 == 0
             and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0 and gate_up.shape[0] <= 4096)
 
 
@@ -1541,8 +1541,8 @@ def _routed_plan_ints(pairs: int, experts: int) -> int:
 def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accumulate=False, identity: int = 0,
                  limit: float = 0.0, beta: float = 1.0, shift: float = 0.0):
     """The routed feed-forward for many rows of bfloat16: the (row, choice) pairs are sorted by expert on the device, an
-    expert's pairs run in tiles of 128 rows on the tensor cores (TMA + tcgen05; gate and up with the gated activation in one
-    kernel, then down), and a row's choices are summed in their order.  ``out`` 32-bit ``[rows, width]``, overwritten or, with
+    expert's pairs run in tiles of 128 rows on the tensor cores (TMA + tcgen05, or mma.sync without ``USE_TCGEN05``; gate and
+    up with the gated activation in one kernel, then down), and a row's choices are summed in their order.  ``out`` 32-bit ``[rows, width]``, overwritten or, with
     ``accumulate``, added to.  Nothing is read back to the host: it can be captured.  ``identity``: how many choices beyond
     the experts are identity experts (the row itself times the weight); ``limit``, ``beta``, ``shift``: as in ``gate_mul``."""
     _need_cuda(h, gate_up, down, ids, weights, out)
@@ -1559,7 +1559,8 @@ def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accu
                                      _ptr(plan), _ptr(x), _ptr(hidden), _ptr(y), _ptr(out), c_int(out.stride(0)), c_int(rows),
                                      c_int(W), c_int(F), c_int(E), c_int(top), c_int(ACT[act]),
                                      c_int(1 if weight_on_input else 0), c_int(1 if accumulate else 0), _stream(),
-                                     c_float(limit), c_float(beta), c_float(shift), _ptr(tcgen05_error_flag(h.device)))
+                                     c_float(limit), c_float(beta), c_float(shift), _ptr(tcgen05_error_flag(h.device)),
+                                     c_int(1 if USE_TCGEN05 else 0))
     _check(st, "routed_tiles", f"rows={rows} width={W} inner={F} experts={E} top={top}", launches=5)
 
 

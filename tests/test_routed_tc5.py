@@ -36,3 +36,11 @@ def test_tiles(ops, rows, W, F, E, top, weight_on_input):
             ref[r] += (a @ dn[e].double().t()) * (1 if weight_on_input else w)
     assert (out.double().cpu() - ref).abs().max() < 2 ** -7 * max(1.0, ref.abs().max())
     ops.raise_if_kernel_errors()
+
+
+@pytest.mark.parametrize("rows,W,F,E,top", [(300, 264, 136, 3, 2), (33, 1032, 264, 5, 3), (129, 8, 8, 4, 2), (400, 320, 72, 40, 2)])
+def test_tiles_without_tcgen05(ops, monkeypatch, rows, W, F, E, top):
+    """With tcgen05 switched off the rows still go sorted by expert, on mma.sync tiles (128 rows, 64 columns, K in pieces of 32)."""
+    monkeypatch.setattr(ops, "USE_TCGEN05", False)
+    test_tiles(ops, rows, W, F, E, top, True)
+    test_tiles(ops, rows, W, F, E, top, False)
