@@ -51,34 +51,24 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two neighbouring values into three bfloat16 parts each, `part` elements apart.  An infinite value (or none) is its first part
-// alone: infinity less infinity would be no number; a value that only rounds to infinity has the largest bfloat16 as its first.
+// Two neighbouring values into three bfloat16 parts each, `part` elements apart.  (What is infinite has rests that are no numbers: it
+// stays not finite, and so does every sum it enters, which are those it enters in the walk row by row.)
 __device__ __forceinline__ void store_parts(__nv_bfloat16* at, int part, float v0, float v1) {
-  __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
-  float r0 = v0 - __low2float(b), r1 = v1 - __high2float(b);
-  const uint32_t bits = *reinterpret_cast<const uint32_t*>(&b);
-  if ((bits & 0x7F80u) == 0x7F80u || (bits & 0x7F800000u) == 0x7F800000u) {
-    constexpr float TOP = 3.3895313892515355e38f;
-    const bool f0 = fabsf(v0) < INFINITY, f1 = fabsf(v1) < INFINITY;
-    b = __floats2bfloat162_rn(f0 ? fminf(fmaxf(v0, -TOP), TOP) : v0, f1 ? fminf(fmaxf(v1, -TOP), TOP) : v1);
-    r0 = f0 ? v0 - __low2float(b) : 0.f;
-    r1 = f1 ? v1 - __high2float(b) : 0.f;
-  }
-  *reinterpret_cast<__nv_bfloat162*>(at) = b;
 #pragma unroll
-  for (int i = 1; i < 3; ++i) {
-    b = __floats2bfloat162_rn(r0, r1);
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
     *reinterpret_cast<__nv_bfloat162*>(at + i * part) = b;
-    r0 -= __low2float(b);
-    r1 -= __high2float(b);
+    v0 -= __low2float(b);
+    v1 -= __high2float(b);
   }
 }
-// Whether one of the eight bfloat16 of a fragment is infinite or no number.
+// Whether one of the eight bfloat16 of a fragment is infinite or no number: 0 times it is no number.
 __device__ __forceinline__ bool not_finite(const uint32_t (&r)[4]) {
-  bool bad = false;
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+  __nv_bfloat162 s = zero;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) bad |= (r[i] & 0x7F80u) == 0x7F80u || (r[i] & 0x7F800000u) == 0x7F800000u;
-  return bad;
+  for (int i = 0; i < 4; ++i) s = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&r[i]), zero, s);
+  return (*reinterpret_cast<const uint32_t*>(&s) & 0x7FFF7FFFu) != 0;
 }
 
 template <int N>
