@@ -1412,6 +1412,14 @@ SCAN_CHUNKS_FROM = 33           # rows of a segment from which it goes 64 rows a
 SCAN_PIECE_ROWS = 128           # rows of a piece
 SCAN_PIECES_FROM = 384          # the longest segment of a step from which segments are cut
 SCAN_PIECES_MAX_STATE = 200_000  # state elements of a step up to which they are
+# ... and up to which long segments go in pieces, not 64 rows at a time: chunks follow one another whatever the state's size (65 to
+# 82 us for 1,024 rows), pieces do not.  us, pieces -> chunks: 8 k elements 512 rows 44 -> 35, 1,024 rows 51 -> 67, 2,048 rows 66 -> 133;
+# 16 k 1,024 rows 64 -> 68 (76 -> 84 with 128 states), 2,048 rows 74 -> 133; 33 k 2,048 rows 139 -> 133.
+SCAN_PIECES_OVER_CHUNKS = 20_000
+
+
+def _pieces_over_chunks(state_elements: int, longest: int) -> bool:
+    return state_elements <= SCAN_PIECES_OVER_CHUNKS and longest >= 450 + state_elements // 32
 
 
 def ssm_scan(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, seg_slot, cu_rows, n_segments, heads, head_dim, n_state,
@@ -1422,7 +1430,7 @@ def ssm_scan(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, seg_slot, cu_rows
     step sizes are columns ``dt_off ..`` of ``proj``; ``y`` ``[T, heads * head_dim]`` 32-bit.
 
     Segments of ``SCAN_CHUNKS_FROM`` rows and more of bfloat16 with heads of a multiple of 32 columns and 64 or 128 states go
-    64 rows at a time as matrix products (32-bit values in three bfloat16 parts).  Otherwise a segment's rows are walked in
+    64 rows at a time as matrix products (32-bit values in three bfloat16 parts; not a long segment of few states).  Otherwise a segment's rows are walked in
     order.  Where the step's longest segment (``max_seg_rows``) is long and the step's
     states are few, segments are cut into pieces of ``piece_rows`` rows that run side by side: every piece's end
     state from zero, then the start states one after the other (S_next = S + expm1(sum of log-decays) S + end), then
@@ -1435,7 +1443,8 @@ def ssm_scan(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, seg_slot, cu_rows
     assert all(t.dtype == torch.float32 and t.numel() == heads for t in (dt_bias, a_log, d_skip))
     longest = int(max_seg_rows) if max_seg_rows is not None else 0
     below = 0
-    if (piece_rows is None and longest >= SCAN_CHUNKS_FROM and xbc.dtype == torch.bfloat16 and head_dim % 32 == 0 and n_state in (64, 128)
+    state_elements = n_segments * heads * head_dim * n_state
+    if (piece_rows is None and longest >= SCAN_CHUNKS_FROM and not _pieces_over_chunks(state_elements, longest) and xbc.dtype == torch.bfloat16 and head_dim % 32 == 0 and n_state in (64, 128)
             and xbc.stride(0) % 8 == 0 and xbc.data_ptr() % 16 == 0 and y.stride(0) % 2 == 0 and y.data_ptr() % 8 == 0):
         below, piece_rows = SCAN_CHUNKS_FROM, 0
         st = kernels().cbis_ssm_chunks(_ptr(xbc), c_int(xbc.stride(0)), _ptr(proj), c_int(proj.stride(0)), c_int(dt_off),
@@ -1446,7 +1455,7 @@ def ssm_scan(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, seg_slot, cu_rows
         if n_segments == 1:
             return
     if piece_rows is None:
-        few = n_segments * heads * head_dim * n_state <= SCAN_PIECES_MAX_STATE
+        few = state_elements <= SCAN_PIECES_MAX_STATE
         piece_rows = SCAN_PIECE_ROWS if (few and longest >= SCAN_PIECES_FROM) else 0
     n_pieces = -(-longest // piece_rows) if piece_rows and longest > piece_rows else 1
     ends = logs = None

@@ -80,3 +80,21 @@ def test_an_infinite_x_reaches_its_own_column_from_its_own_row_on(value, at):
     assert not torch.isfinite(y1[at:, col]).any() and not torch.isfinite(s1[col]).any()
     y1[at:, col], s1[col] = y0[at:, col], s0[col]
     assert (y1 - y0).abs().max() <= 2e-6 * y0.abs().max() and (s1 - s0).abs().max() <= 2e-6 * s0.abs().max()
+
+
+@pytest.mark.parametrize("H,P,N,rows,launches", [(2, 64, 64, 1100, 3), (2, 64, 64, 640, 1), (4, 32, 128, 1000, 3), (8, 64, 64, 1500, 1)])
+def test_long_segments_of_few_states_go_in_pieces(H, P, N, rows, launches):
+    """8,192 and 16,384 state elements from some 700 and 960 rows on: three launches side by side; fewer rows or more states: one
+    kernel, chunk after chunk.  Sums of up to 1,100 32-bit terms around 1, twice over: 4e-6 of the largest."""
+    from cbis_b200.kernels import ops
+    g = torch.Generator().manual_seed(rows)
+    xbc, raw = torch.randn(rows, H * P + 2 * N, generator=g).bfloat16(), torch.randn(rows, H, generator=g).bfloat16()
+    a_log, dt_bias, d_skip = torch.randn(H, generator=g), torch.randn(H, generator=g) - 1.0, torch.randn(H, generator=g)
+    state, y = torch.zeros(1, H * P * N, device="cuda"), torch.empty(rows, H * P, device="cuda")
+    before = ops.launch_count()
+    ops.ssm_scan(xbc.cuda(), raw.cuda(), 0, dt_bias.cuda(), a_log.cuda(), d_skip.cuda(), state, torch.zeros(1, dtype=torch.int32, device="cuda"),
+                 torch.tensor([0, rows], dtype=torch.int32, device="cuda"), 1, H, P, N, 1, y, max_seg_rows=rows)
+    assert ops.launch_count() - before == launches
+    ref, S = walk(xbc.double(), raw.double(), a_log.double(), dt_bias.double(), d_skip.double(), H, P, N, 1)
+    assert (y.double().cpu() - ref).abs().max() < 4e-6 * ref.abs().max()
+    assert (state.view(H, P, N).double().cpu() - S).abs().max() < 4e-6 * S.abs().max()
