@@ -193,10 +193,10 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 // loads, all in flight at once, and every thread then walks its piece from left to right with one fused
 // multiply-add per element: the same order as the tiled kernel, hence the same bits, so that a token decoded
 // alone and the same token inside a prompt portion still agree exactly.
-// With 16-byte aligned rows (linear_f32_few_rows_kernel<true>) up to four pieces are on their way at once, the weights' since
+// With 16-byte aligned rows (STAGES > 0) up to STAGES pieces are on their way at once, the weights' since
 // before the wait for the kernel ahead: piece by piece, each a trip to L2 with nothing else to do, the products of a
 // 256-wide model's decode step took 6.7 us on average; 5.2 so, 4.8 with the blocks spread evenly (common.cuh).
-constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4, FR_STAGES = 4;
+constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4, FR_STAGE_BYTES = 32 * FR_PITCH * (int)sizeof(float);
 __device__ __forceinline__ float few_rows_walk(const float* a, const float* w, int kc, float acc) {
   int k = 0;
 #pragma unroll 8
@@ -210,7 +210,7 @@ __device__ __forceinline__ float few_rows_walk(const float* a, const float* w, i
   for (; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
   return acc;
 }
-template <bool ALIGNED>
+template <int STAGES>
 __global__ void __launch_bounds__(256)
 linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                            int M, int N, int K, int act, int lda, int ldc) {
@@ -219,9 +219,9 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
   const int tid = threadIdx.x;
   const int m = tid & 15, c = tid >> 4, n0 = blockIdx.x * 16, n = n0 + c;
   float acc = 0.f;
-  if constexpr (ALIGNED) {
-    const int n_p = (K + FR_KC - 1) / FR_KC, stages = min(n_p, FR_STAGES);
-    auto a_of = [&](int p) { return fr_smem + (size_t)(p % stages) * 32 * FR_PITCH; };
+  if constexpr (STAGES > 0) {
+    const int n_p = (K + FR_KC - 1) / FR_KC;
+    auto a_of = [&](int p) { return fr_smem + (size_t)(p % STAGES) * 32 * FR_PITCH; };
     auto load = [&](int p, const float* src, int ld, int rows, float* dst) {      // 16 rows of 256: rows past the end are zeros
       for (int i = tid; i < 16 * (FR_KC / 4); i += 256) {
         const int r = i / (FR_KC / 4), k = (i % (FR_KC / 4)) * 4;
@@ -230,22 +230,22 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
       }
     };
     const float* w0 = W + (size_t)n0 * K;
-    for (int p = 0; p < stages; ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+    for (int p = 0; p < min(n_p, STAGES); ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
     const float b = bias && n < N ? bias[n] : 0.f;
     pdl_wait();  // A comes from the kernel before
-    for (int p = 0; p < FR_STAGES; ++p) {
-      if (p < stages) load(p, A, lda, M, a_of(p));
+    for (int p = 0; p < STAGES; ++p) {
+      if (p < n_p) load(p, A, lda, M, a_of(p));
       cp_async_commit();
     }
     for (int p = 0; p < n_p; ++p) {
-      cp_async_wait<FR_STAGES - 1>();
+      cp_async_wait<STAGES - 1>();
       __syncthreads();
       const float* a = a_of(p);
       acc = few_rows_walk(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
-      if (p + stages < n_p) {
+      if (p + STAGES < n_p) {
         __syncthreads();
-        load(p + stages, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
-        load(p + stages, A, lda, M, a_of(p));
+        load(p + STAGES, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+        load(p + STAGES, A, lda, M, a_of(p));
       }
       cp_async_commit();
     }
@@ -318,10 +318,14 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
   }
   if (w_is_nk) {   // decoding: one thread per output, 16 outputs (rows) x 2 columns per warp, 8 warps per block
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
-    auto kern = aligned ? linear_f32_few_rows_kernel<true> : linear_f32_few_rows_kernel<false>;
-    const int pieces = (K + FR_KC - 1) / FR_KC, stages = !aligned ? 1 : (pieces < FR_STAGES ? pieces : FR_STAGES);
+    const int pieces = (K + FR_KC - 1) / FR_KC, per_sm = ((N + 15) / 16 + 147) / 148;
+    // as long a ring as lets all of an SM's blocks (up to the six that one stage allows) run side by side: 16 rows, K = 2,048, four
+    // stages -> this rule: N = 6,144 61 us -> 46, 50,257 442 -> 307; N = 2,304 with one stage 24, with two 21
+    const int ring = per_sm <= 1 ? 4 : (per_sm <= 3 ? 2 : 1), stages = !aligned ? 1 : (pieces < ring ? pieces : ring);
+    auto kern = !aligned ? linear_f32_few_rows_kernel<0> : (ring == 4 ? linear_f32_few_rows_kernel<4>
+                         : (ring == 2 ? linear_f32_few_rows_kernel<2> : linear_f32_few_rows_kernel<1>));
     size_t smem;
-    cudaError_t e = spread_evenly(kern, (N + 15) / 16, (size_t)stages * 32 * FR_PITCH * sizeof(float), &smem);
+    cudaError_t e = spread_evenly(kern, (N + 15) / 16, (size_t)stages * FR_STAGE_BYTES, &smem);
     if (e != cudaSuccess) return (int)e;
     return (int)launch_pdl(kern, dim3((N + 15) / 16), dim3(256), smem, st, A, W, bias, C, M, N, K, act, lda, ldc);
   }
