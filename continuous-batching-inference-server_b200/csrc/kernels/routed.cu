@@ -17,10 +17,10 @@ namespace cbis {
 
 constexpr int kScoreSigmoid = 0, kScoreSoftmax = 1;
 
-// grid (rows), a warp for each router row up to 32; shared: 2 (E + 1) floats.  ids [rows, top] int32, weights [rows, top] float.  correction (may
+// grid (rows), blocks of whole warps; shared: 2 (E + 1) floats.  ids [rows, top] int32, weights [rows, top] float.  correction (may
 // be null): [E], added to the scores for the choice.  side (may be null): [rows], the sigmoid of router row E's logit.
-template <typename TT>
-__global__ void __launch_bounds__(1024)
+template <typename TT, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 route_topk_kernel(const TT* h, int h_ld, const TT* __restrict__ router, int* ids, float* weights, int W, int E, int top,
                   int score, int renormalize, float renorm_eps, float weight_scale, const float* __restrict__ correction,
               float* side) {
@@ -32,7 +32,7 @@ route_topk_kernel(const TT* h, int h_ld, const TT* __restrict__ router, int* ids
   const TT* hr = h + (size_t)r * h_ld;
   constexpr int V = 16 / (int)sizeof(TT);      // elements of a 16-byte load
   const bool vec = W % V == 0 && !(((uintptr_t)hr | (uintptr_t)router) & 15);
-  for (int e = warp; e < E + (side ? 1 : 0); e += blockDim.x >> 5) {
+  for (int e = warp; e < E + (side ? 1 : 0); e += THREADS == 256 ? 8 : blockDim.x >> 5) {
     const TT* wr = router + (size_t)e * W;
     float acc = 0.f;
     if (vec) {
@@ -207,18 +207,25 @@ CBIS_EXPORT int cbis_route_topk(const void* h, int h_ld, const void* router, int
   if (E > 6000) return CBIS_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = (size_t)2 * (E + 1) * sizeof(float);
-  // few rows (decoding): a warp for every router row, so that no warp takes two rows of the router one after the other; many
-  // rows fill the SMs anyway, with eight warps each
-  const int warps = rows > 4 * 148 ? 8 : (E + 1 < 8 ? 8 : (E + 1 > 32 ? 32 : E + 1));
-  const dim3 block(32 * warps);
-  if (dtype == CBIS_F32)
-    return (int)launch_pdl(route_topk_kernel<float>, dim3(rows), block, smem, st, (const float*)h, h_ld,
-                           (const float*)router, ids, weights, W, E, top, score, renormalize, renorm_eps, weight_scale,
-                           correction, side);
-  if (dtype == CBIS_BF16)
-    return (int)launch_pdl(route_topk_kernel<__nv_bfloat16>, dim3(rows), block, smem, st, (const __nv_bfloat16*)h, h_ld,
-                           (const __nv_bfloat16*)router, ids, weights, W, E, top, score, renormalize, renorm_eps,
-                           weight_scale, correction, side);
+  // A warp for every router row (up to 32), so that no warp takes two of them one after the other, while the SMs hold the warps
+  // of all rows at once, or nearly so; else eight warps a row (of more registers each, hence a kernel of its own).  Eight warps -> more
+  // at width 2,048: 148 rows, 64 experts 14.1 -> 9.6 us; 300 rows, 24 experts 9.4 -> 9.8, 64 experts 23.6 -> 18.7; 592 rows, 64
+  // experts 20.2 -> 23.2, 256 experts 71 -> 63.
+  const int n = E + (side ? 1 : 0), warps = n < 32 ? n : 32, per_sm = (rows + 147) / 148;
+  const bool many = n > 8 && ((per_sm <= 3 && (per_sm * warps <= 64 || n >= 48)) || (per_sm == 4 && n >= 128));
+#define CBIS_ROUTE(TT, THREADS)                                                                                           \
+  return (int)launch_pdl(route_topk_kernel<TT, THREADS>, dim3(rows), dim3(THREADS == 256 ? 256 : 32 * warps), smem, st, \
+                         (const TT*)h, h_ld, (const TT*)router, ids, weights, W, E, top, score, renormalize, renorm_eps,  \
+                         weight_scale, correction, side)
+  if (dtype == CBIS_F32) {
+    if (many) CBIS_ROUTE(float, 1024);
+    CBIS_ROUTE(float, 256);
+  }
+  if (dtype == CBIS_BF16) {
+    if (many) CBIS_ROUTE(__nv_bfloat16, 1024);
+    CBIS_ROUTE(__nv_bfloat16, 256);
+  }
+#undef CBIS_ROUTE
   return CBIS_ERR_BAD_DTYPE;
 }
 
