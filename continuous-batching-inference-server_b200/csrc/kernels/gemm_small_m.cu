@@ -70,7 +70,7 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
                                                   int N, int K, int act, const void* next_w,
                                                   unsigned long long next_bytes, int ksplit, int accumulate, int group_n, int act_from,
                                                   const GatedEpilogue* glu = nullptr) {
-  static_assert(!GLU || NT == 2, "a block of the gated form takes 8 gate and 8 up columns");
+  static_assert(!GLU || (NT == 2 && !CLUSTER), "a block of the gated form takes 8 gate and 8 up columns and all of K");
   extern __shared__ float red[];  // [SM_WARPS][MT*16][NT*8 + 1], then [ksplit - 1][MT*16 * NT*8] for the other blocks' sums
   constexpr int RS = NT * 8 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -215,8 +215,6 @@ __device__ __forceinline__ void gemm_small_m_body(const __nv_bfloat16* A, int ld
       for (int j = 0; j < 2; ++j) {
 #pragma unroll
         for (int w = 0; w < SM_WARPS; ++w) v[j] += red[((size_t)w * (MT * 16) + m) * RS + j * 8 + c];
-        if constexpr (CLUSTER)
-          for (int r = 1; r < ksplit; ++r) v[j] += others[(size_t)(r - 1) * (MT * 16) * (NT * 8) + m * (NT * 8) + j * 8 + c];
       }
       const float gate = to_f32(__float2bfloat16_rn(v[0] + bias0)), up = to_f32(__float2bfloat16_rn(v[1] + bias1));
       float o = gated_product(gate, up, act, glu->limit, glu->beta, glu->shift);
@@ -266,13 +264,13 @@ gemm_small_m_low8_ksplit_kernel(const __nv_bfloat16* A, int lda, const __nv_bflo
   gemm_small_m_body<MT, NT, UNROLL, true, TO, true>(A, lda, W, bias, C, ldc, M, N, K, act, next_w, next_bytes, ksplit, accumulate, group_n, act_from);
 }
 
-// The gated form: up to 8 rows with K over the blocks of a cluster or not, and up to 16 rows.
-template <bool LOW8, bool CLUSTER>
+// The gated form: up to 8 rows in 64 registers, or up to 16 rows.
+template <bool LOW8>
 __global__ void __launch_bounds__(SM_WARPS * 32, LOW8 ? 4 : 3)
 gemm_small_m_gated_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                           __nv_bfloat16* __restrict__ C, int ldc, int M, int F, int K, int act, const void* next_w,
-                          unsigned long long next_bytes, int ksplit, const GatedEpilogue glu) {
-  gemm_small_m_body<1, 2, 4, LOW8, __nv_bfloat16, CLUSTER, false, false, true>(A, lda, W, bias, C, ldc, M, F, K, act, next_w, next_bytes, ksplit, 0, 0, 0, &glu);
+                          unsigned long long next_bytes, const GatedEpilogue glu) {
+  gemm_small_m_body<1, 2, 4, LOW8, __nv_bfloat16, false, false, false, true>(A, lda, W, bias, C, ldc, M, F, K, act, next_w, next_bytes, 1, 0, 0, 0, &glu);
 }
 
 template <int MT, int NT, int UNROLL, bool LOW8, typename TO, bool TILES = false>
@@ -391,28 +389,10 @@ CBIS_EXPORT int cbis_gemm_small_m_gated_bf16(const void* A, int lda, const void*
   if (M > 16 || K <= 0 || K % 8 || lda < K || ldc < F) return CBIS_ERR_BAD_SIZE;
   if (lda % 8 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)next_w & 15)) return CBIS_ERR_ALIGNMENT;
   const GatedEpilogue glu = {limit, beta, shift, row_gate};
-  const int tiles = (F + 7) / 8, nkb = (K + 31) / 32;
-  int ks = 1;      // as dispatch_small_m splits K: few columns, one round of K blocks a warp
-  if (M <= 8 && ksplit_enabled())
-    while (ks < 4 && tiles * ks * 2 <= 4 * 148 && nkb >= SM_WARPS * 4 * ks * 2) ks *= 2;
-  const size_t smem = ((size_t)SM_WARPS * 16 * 17 + (size_t)(ks - 1) * 16 * 16) * sizeof(float);
+  const int tiles = (F + 7) / 8;
+  const size_t smem = (size_t)SM_WARPS * 16 * 17 * sizeof(float);
   // (more blocks than four an SM: the general form, three an SM, is the faster one, 11.5 us against 13.0 on 5,440 x 2,048)
-  auto kern = ks > 1 ? gemm_small_m_gated_kernel<true, true>
-                     : (M <= 8 && tiles > 3 * 148 && tiles <= 4 * 148 ? gemm_small_m_gated_kernel<true, false> : gemm_small_m_gated_kernel<false, false>);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * ks));
-  cfg.blockDim = dim3(SM_WARPS * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled();
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)ks;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = ks > 1 ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)W, bias, (__nv_bfloat16*)C, ldc, M, F,
-                                 K, act, next_w, next_bytes, ks, glu);
+  auto kern = M <= 8 && tiles > 3 * 148 && tiles <= 4 * 148 ? gemm_small_m_gated_kernel<true> : gemm_small_m_gated_kernel<false>;
+  return (int)launch_pdl(kern, dim3(tiles), dim3(SM_WARPS * 32), smem, (cudaStream_t)stream, (const __nv_bfloat16*)A, lda,
+                         (const __nv_bfloat16*)W, bias, (__nv_bfloat16*)C, ldc, M, F, K, act, next_w, next_bytes, glu);
 }

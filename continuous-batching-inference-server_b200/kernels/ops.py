@@ -244,6 +244,16 @@ def gated_linear_takes(x, w_gate_up) -> bool:
             and x.data_ptr() % 16 == 0)
 
 
+def gated_linear_pays(rows: int, inner: int, K: int) -> bool:
+    """Whether ``gated_linear`` is faster for these sizes than the product and ``gate_mul``, whose sums it has, bit for bit.  Not
+    where the product would split K over the blocks of a cluster (up to 8 rows, few columns, a long K): at inner 1,408 and
+    K 2,048 the two take 5.5 us for 6 rows and a gated form that splits K too 6.1; at 1,024 and 4,096 5.8, and 8.4 for one that
+    does not.  Not for 110 MB of weights and more, where a block's columns lie too far apart: inner 11,008 and K 4,096, 16 rows,
+    42.9 against 44.4 us.  Elsewhere it is the faster one: inner 5,440 and K 2,048, 4 rows, 13.2 against 11.9."""
+    n = 2 * inner
+    return not (rows <= 8 and 64 <= n < 148 * 2 * 16 and K > 63 * 32) and 2 * n * K < 110e6
+
+
 def gated_linear(x, w_gate_up, bias, act, out, row_gate=None, limit: float = 0.0, beta: float = 1.0, shift: float = 0.0):
     """out = act(x @ Wg^T + bg) * (x @ Wu^T + bu) for up to 16 rows of bfloat16: the gated product of two products with the
     rows of ``w_gate_up`` (the gate's, then the up projection's), whose sums are rounded to bfloat16 as ``linear`` does.  ``limit``,

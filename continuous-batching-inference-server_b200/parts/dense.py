@@ -111,7 +111,7 @@ class GatedFeedForward(FeedForward):
     def _inside(self, h, row_gate=None):
         F = self.inner
         a = torch.empty((h.shape[0], F), dtype=h.dtype, device=h.device)
-        if ops.gated_linear_takes(h, self.w_gate_up):       # a few rows: one kernel
+        if ops.gated_linear_takes(h, self.w_gate_up) and ops.gated_linear_pays(h.shape[0], F, h.shape[1]):      # a few rows: one kernel
             ops.gated_linear(h, self.w_gate_up, self.b_gate_up, self.activation, a, row_gate=row_gate, **self.shape)
             return a
         gu = ops.linear(h, self.w_gate_up, self.b_gate_up)
