@@ -293,8 +293,9 @@ paged_decode_tc_kernel(const __nv_bfloat16* qkv, int ld, int k_off, int v_off, _
 
 // The plan of a step's decoding rows for one window: how many keys a piece holds, then every row's pieces, the longest
 // pieces first (blocks start in this order, so the short ones fill the gaps at the end).  A head's pieces: `fit` at most
-// where the rows leave room for that (one round of blocks over the SMs: a piece more than they hold would cost a second
-// round), else about `fit` in all.  No piece is shorter than `round` keys and no row has more than 32.
+// if the rows are no more than that (one round of blocks over the SMs: a piece more than they hold would cost a second
+// round), else rows + `fit` at most.  No piece is shorter than `round` keys and no row has more than 32.  Rows that are at most one
+// round longer than such a piece stay whole, all of them: the merge of a row's pieces takes 2.5 us, a round 1.2 to 1.8.
 // One block; it lets its successor start only when it ends: an attention kernel reads its plan before it waits for
 // the kernels ahead.
 constexpr int PLAN_THREADS = 256;
@@ -323,15 +324,15 @@ decode_plan_kernel(const int* row_seq, const int* positions, int rows, int windo
   atomicMax(&s_longest, longest);
   __syncthreads();
   if (tid < 32) {
-    // lane i tries i rounds more than an even share: the first that fits
-    const long long even = max((s_total + fit - 1) / fit, (long long)(s_longest + 31) / 32);
-    const int keys0 = (int)((even + round - 1) / round) * round;
-    const int keys = max(keys0, round) + lane * round;
+    // lane i tries i steps more than an even share, the last one the longest row whole: the first that fits
+    const long long even = min(max((s_total + fit - 1) / fit, (long long)(s_longest + 31) / 32), (long long)s_longest);
+    const int keys0 = max((int)((even + round - 1) / round), 1) * round;
+    const int keys = keys0 + lane * max((s_longest - keys0 + 31 * round - 1) / (31 * round), 1) * round;
     int n = 0;
     for (int r = 0; r < rows; ++r) n += max((len_of[r] + keys - 1) / keys, 1);
     const unsigned ok = __ballot_sync(0xffffffffu, n <= fit);
-    const int pick = rows > fit ? 0 : (ok ? __ffs(ok) - 1 : 31);
-    if (lane == pick) s_keys = keys;
+    const int pick = rows > fit ? 0 : __ffs(ok) - 1;
+    if (lane == pick) s_keys = s_longest <= keys + round ? max(s_longest, keys) : keys;
   }
   __syncthreads();
   for (int r = tid; r < rows; r += PLAN_THREADS) n_of[r] = max((len_of[r] + s_keys - 1) / s_keys, 1);
@@ -461,7 +462,7 @@ CBIS_EXPORT int cbis_paged_decode_bf16(const void* qkv, int ld, int k_off, int v
 }
 
 // The plan for cbis_paged_decode_bf16 with nsplit 0: `plan` takes `most` entries of 16 bytes, of which at most
-// rows + fit are pieces (most >= that, or >= rows times the most pieces a row can have).  rows <= PLAN_MAX_ROWS.
+// rows + fit are pieces, or fit if rows <= fit (most >= that, or >= rows times the most pieces a row can have).  rows <= PLAN_MAX_ROWS.
 CBIS_EXPORT int cbis_decode_plan(const int* row_seq, const int* positions, int rows, int window, int keep, int fit, int round,
                                  void* plan, int most, void* stream) {
   if (rows <= 0) return CBIS_OK;

@@ -57,8 +57,8 @@ def _decode_cut(ctx, v_pages, n_head, hd, vd, ps, window, extra):
     counters).  Where the kernel can, by the rows' own lengths, in pieces of about one size; the plan of that is made once
     for all layers of the step that cut alike."""
     nd, limit = ctx.n_decode, ctx.ctx_limit
-    # (a single row is cut evenly in any case; its pieces need no plan, whose lookup cost 1.5 us a layer)
-    if 1 < nd <= 4096 and ops.decode_in_pieces(v_pages, hd, ps, **extra):
+    nsplit = ops.decode_splits(nd, n_head, limit)
+    if ops.decode_plan_pays(nd, n_head, limit, nsplit) and ops.decode_in_pieces(v_pages, hd, ps, **extra):
         key = ("decode_plan", n_head, hd, window, extra.get("keep", 0))
         plan = ctx.shared.get(key)
         if plan is None:
