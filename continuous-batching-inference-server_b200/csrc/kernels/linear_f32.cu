@@ -220,8 +220,8 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
   const int m = tid & 15, c = tid >> 4, n0 = blockIdx.x * 16, n = n0 + c;
   float acc = 0.f;
   if constexpr (STAGES > 0) {
-    const int n_p = (K + FR_KC - 1) / FR_KC;
-    auto a_of = [&](int p) { return fr_smem + (size_t)(p % STAGES) * 32 * FR_PITCH; };
+    const int n_p = (K + FR_KC - 1) / FR_KC, stages = min(n_p, STAGES);
+    auto a_of = [&](int p) { return fr_smem + (size_t)(p % stages) * 32 * FR_PITCH; };
     auto load = [&](int p, const float* src, int ld, int rows, float* dst) {      // 16 rows of 256: rows past the end are zeros
       for (int i = tid; i < 16 * (FR_KC / 4); i += 256) {
         const int r = i / (FR_KC / 4), k = (i % (FR_KC / 4)) * 4;
@@ -230,11 +230,11 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
       }
     };
     const float* w0 = W + (size_t)n0 * K;
-    for (int p = 0; p < min(n_p, STAGES); ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+    for (int p = 0; p < stages; ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
     const float b = bias && n < N ? bias[n] : 0.f;
     pdl_wait();  // A comes from the kernel before
     for (int p = 0; p < STAGES; ++p) {
-      if (p < n_p) load(p, A, lda, M, a_of(p));
+      if (p < stages) load(p, A, lda, M, a_of(p));
       cp_async_commit();
     }
     for (int p = 0; p < n_p; ++p) {
@@ -242,10 +242,10 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
       __syncthreads();
       const float* a = a_of(p);
       acc = few_rows_walk(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
-      if (p + STAGES < n_p) {
+      if (p + stages < n_p) {
         __syncthreads();
-        load(p + STAGES, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
-        load(p + STAGES, A, lda, M, a_of(p));
+        load(p + stages, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+        load(p + stages, A, lda, M, a_of(p));
       }
       cp_async_commit();
     }
