@@ -295,7 +295,8 @@ paged_decode_tc_kernel(const __nv_bfloat16* qkv, int ld, int k_off, int v_off, _
 // pieces first (blocks start in this order, so the short ones fill the gaps at the end).  A head's pieces: `fit` at most
 // if the rows are no more than that (one round of blocks over the SMs: a piece more than they hold would cost a second
 // round), else rows + `fit` at most.  No piece is shorter than `round` keys and no row has more than 32.  Rows that are at most one
-// round longer than such a piece stay whole, all of them: the merge of a row's pieces takes 2.5 us, a round 1.2 to 1.8.
+// round longer than such a piece (two, if there are more rows than that) stay whole, all of them: the merge of a row's pieces takes 2.5
+// us, a round 1.2 to 1.8, and with more rows than fit side by side the pieces only make the second round of blocks longer.
 // One block; it lets its successor start only when it ends: an attention kernel reads its plan before it waits for
 // the kernels ahead.
 constexpr int PLAN_THREADS = 256;
@@ -332,7 +333,7 @@ decode_plan_kernel(const int* row_seq, const int* positions, int rows, int windo
     for (int r = 0; r < rows; ++r) n += max((len_of[r] + keys - 1) / keys, 1);
     const unsigned ok = __ballot_sync(0xffffffffu, n <= fit);
     const int pick = rows > fit ? 0 : __ffs(ok) - 1;
-    if (lane == pick) s_keys = s_longest <= keys + round ? max(s_longest, keys) : keys;
+    if (lane == pick) s_keys = s_longest <= keys + (rows > fit ? 2 : 1) * round ? max(s_longest, keys) : keys;
   }
   __syncthreads();
   for (int r = tid; r < rows; r += PLAN_THREADS) n_of[r] = max((len_of[r] + s_keys - 1) / s_keys, 1);

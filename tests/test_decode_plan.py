@@ -23,6 +23,8 @@ def test_the_plan_covers_every_key_once(ops, rows, n_head, hd, longest):
     seq = torch.arange(rows, dtype=torch.int32)
     if rows > 2:
         seq[2] = -1
+    if rows == 24:                                                        # an even share is one round of keys, the longest row three
+        pos[1:] //= 2
     if longest == 30000:                                                  # one place more than rows, and rows of more than half the
         pos[1:] = longest // 2 + 1                                        # longest: hardly any cut is few enough
     plan = ops.decode_plan(dev(seq), dev(pos), rows, n_head, longest, hd)
