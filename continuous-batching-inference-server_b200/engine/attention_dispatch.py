@@ -64,7 +64,6 @@ def _decode_cut(ctx, v_pages, n_head, hd, vd, ps, window, extra):
         if plan is None:
             plan = ctx.shared[key] = ops.decode_plan(ctx.row_seq, ctx.positions, nd, n_head, limit, hd, window, extra.get("keep", 0))
         return (0, plan) + ctx.decode_scratch(n_head * plan.shape[0] * (hd + 2), nd * n_head)
-    nsplit = ops.decode_splits(nd, n_head, limit)
     if nsplit == 1:
         return 1, None, None, None
     return (nsplit, None) + ctx.decode_scratch(ops.decode_scratch_floats(nd, n_head, vd, nsplit), nd * n_head)
@@ -225,7 +224,8 @@ def _plain(ctx, mixer, qkv, cache, view, out, nd, T, hd, ps, k_pages, v_pages, k
                                             ctx.positions[d], out[d], mixer.n_head, mixer.n_kv_head, hd, ps, mixer.scale,
                                             mixer.window, chunks, partial)
             if ctx.n_segments > nd:
-                # (three blocks fit on an SM; pieces for five times as many, so that the last ones leave few SMs idle)
+                # (three blocks fit on an SM at head size 32, two at 48 to 128; pieces for five to eight times as many, so that the
+                # last ones leave few SMs idle: 2,048 rows of 8 heads of 32 110 us with half as many, 91 so; 48 to 96 the same either way)
                 chunks, partial = _key_chunks(ctx, mixer.n_head, nd, T, hd, blocks_per_sm=16)
                 ops.paged_prefill_f32(qkv, k_pages, v_pages, view.block_table, ctx.cu_rows, ctx.seg_start, out, nd,
                                       ctx.n_segments - nd, ctx.max_seg_rows, mixer.n_head, mixer.n_kv_head, hd, ps,

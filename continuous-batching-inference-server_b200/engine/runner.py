@@ -458,7 +458,8 @@ class ModelRunner:
         if len(self._shape_graphs) >= self.max_shape_graphs and not self._takes_a_place(seen):
             return None
         ctx = self.build_context(entries, fixed_shapes=True)
-        # The step itself runs ONCE, launch by launch, with the launches the graph will hold; the capture that
+        # The step itself runs ONCE, launch by launch, with the kernels the graph will hold (which the graph may place on two
+        # branches: decode attention beside a portion's, see attention_dispatch.py); the capture that
         # follows records them without running them, and the recorded step's output buffer takes this run's
         # logits.  (Running it a second time through the fresh graph would be harmless for keys and values,
         # which are written alike both times, but would move a mixer's own per-request state on twice.)
