@@ -92,9 +92,11 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// NK_STAGES pieces are in the ring: a piece of a 32 x 32 tile is multiplied in 0.3 us, a trip to L2 takes 0.7, so with two
+// Five pieces are in the ring: a piece of a 32 x 32 tile is multiplied in 0.3 us, a trip to L2 takes 0.7, so with two
 // buffers a block waited most of its time (the two products of 512 rows with 256 columns, K 256 and 1,024: 55 us on average; 29 with the ring, 14 with the blocks spread evenly as well).
-constexpr int NK_STAGES = 5;
+// Four for the larger tiles, so that three blocks (of 64 x 64) or four fit on an SM: with five, 2048 x 6144 x 2048 took 1,426 us (with
+// two buffers 1,410), 512 x 2048 x 2048 205; with four 1,352 and 151.
+template <int TILE> constexpr int nk_stages = TILE > 32 * 32 ? 4 : 5;
 // A thread owns TM x TN outputs: with more a load from shared memory serves more multiply-adds, with fewer a block has the
 // warps to hide a load's trip.  32 x 64: 4 x 4 (512 x 768 x 256: 14.8 us, 2 x 4: 15.9); 32 x 32, a grid that gives an SM one block:
 // 2 x 2 (512 x 256 x 1024: 20 us, 2 x 4: 28, 4 x 4: 39).
@@ -102,7 +104,7 @@ template <int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                      int M, int N, int K, int act, int lda, int ldc) {
-  constexpr int BK = 32, PITCH = BK + 4, TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
+  constexpr int NK_STAGES = nk_stages<BM * BN>, BK = 32, PITCH = BK + 4, TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
   extern __shared__ __align__(16) float nk_smem[];
   float (*As)[BM][PITCH] = reinterpret_cast<float (*)[BM][PITCH]>(nk_smem);                              // [NK_STAGES][BM][PITCH]
   float (*Ws)[BN][PITCH] = reinterpret_cast<float (*)[BN][PITCH]>(nk_smem + NK_STAGES * BM * PITCH);     // [NK_STAGES][BN][PITCH]
@@ -297,7 +299,7 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
     auto kern = linear_f32_nk_kernel<BM_, BN_, TM_, TN_>;                                                              \
     const dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);                                                         \
     size_t smem;                                                                                                       \
-    cudaError_t e = spread_evenly(kern, (long long)grid.x * grid.y, NK_STAGES * (BM_ + BN_) * 36 * sizeof(float), &smem); \
+    cudaError_t e = spread_evenly(kern, (long long)grid.x * grid.y, nk_stages<BM_ * BN_> * (BM_ + BN_) * 36 * sizeof(float), &smem); \
     if (e != cudaSuccess) return (int)e;                                                                               \
     return (int)launch_pdl(kern, grid, dim3((BM_ / TM_) * (BN_ / TN_)), smem, st, A, W, bias, C, M, N, K, act, lda, ldc); \
   }
