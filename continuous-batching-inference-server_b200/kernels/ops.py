@@ -1567,13 +1567,13 @@ def _routed_plan_ints(pairs: int, experts: int) -> int:
     return int(fn(c_int(pairs), c_int(experts)))
 
 
-def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accumulate=False, limit: float = 0.0,
-                 beta: float = 1.0, shift: float = 0.0):
+def routed_tiles(h, gate_up, down, ids, weights, act, weight_on_input, out, accumulate=False, identity: int = 0,
+                 limit: float = 0.0, beta: float = 1.0, shift: float = 0.0):
     """The routed feed-forward for many rows of bfloat16: the (row, choice) pairs are sorted by expert on the device, an
     expert's pairs run in tiles of 128 rows on the tensor cores (TMA + tcgen05, or mma.sync without ``USE_TCGEN05``; gate and
     up with the gated activation in one kernel, then down), and a row's choices are summed in their order.  ``out`` 32-bit ``[rows, width]``, overwritten or, with
-    ``accumulate``, added to.  Nothing is read back to the host: it can be captured.  A choice beyond the experts is an
-    identity expert (the row itself times the weight).  ``limit``, ``beta``, ``shift``: as in ``gate_mul``."""
+    ``accumulate``, added to.  Nothing is read back to the host: it can be captured.  ``identity``: how many choices beyond
+    the experts are identity experts (the row itself times the weight); every choice beyond the experts is taken for one.  ``limit``, ``beta``, ``shift``: as in ``gate_mul``."""
     _need_cuda(h, gate_up, down, ids, weights, out)
     rows, W = h.shape
     E, F2, _ = gate_up.shape

@@ -101,7 +101,7 @@ class RoutedFeedForward(FeedForward):
         if ops.routed_tiles_takes(h, self.w_gate_up, self.w_down):
             # many rows: sorted by expert, tiles on the tensor cores
             ops.routed_tiles(h, self.w_gate_up, self.w_down, ids, weights, self.activation, self.weight_on_input, out,
-                             accumulate=into is not None, **self.shape)
+                             accumulate=into is not None, identity=self.identity, **self.shape)
         else:
             # a few rows (decoding), and the 32-bit path: every (row, choice) streams its expert's matrices
             hidden = torch.empty((T * self.top, self.inner), dtype=h.dtype, device=h.device)
