@@ -5,7 +5,7 @@
 //   S'  = e^(c_last) S  +  sum over s of B_s (e^(c_last - c_s) dt_s x_s)^T
 // which is what the row-by-row walk computes, in other groups of sums.  The walk is a chain of dependent steps (422 us for
 // 1,500 rows of 64 heads of 64 x 128 on one prompt, a quarter of a microsecond a row, with most of the SM waiting); here
-// the chain is one step per 64 rows, and the same prompt takes 128 us.  Against 64 bits the results are three times as close as
+// the chain is one step per 64 rows, and the same prompt takes 111 us.  Against 64 bits the results are three times as close as
 // the walk's (2.9e-7 of the largest value, the walk 8.8e-7, over segments of 33 to 700 rows).
 //
 // The products run on the tensor cores (mma.sync m16n8k16, 32-bit sums) without giving up 32-bit values: x, B and C are
@@ -15,7 +15,8 @@
 // round it: the first parts' products and the others' are summed apart, and every sum begins at zero and is added to what
 // was there with a rounding of its own, so that few of these cuts fall on a large value.
 //
-// grid (P / 32, heads, segments), 256 threads: a block walks the chunks of one segment for 32 columns of one head's state,
+// grid (P / 32, heads, segments), eight warps and one that works out the next chunk's step sizes and decays (a chain of logarithms,
+// exponentials and shuffles in which the eight would wait: 128 us instead of 111, and 115 instead of 86 for 32 heads of 64 x 64): a block walks the chunks of one segment for 32 columns of one head's state,
 // which stays in registers between chunks (the accumulators of its own update).  155 KB of shared memory at N = 128: one block
 // an SM; the next chunk's rows arrive by cp.async while this one is worked on.
 #include "common.cuh"
@@ -23,7 +24,7 @@
 namespace cbis {
 namespace ssm {
 
-constexpr int Q = 64, PB = 32, THREADS = 256;
+constexpr int Q = 64, PB = 32, WORKERS = 256, THREADS = WORKERS + 32;
 constexpr int MP = Q + 8, XP = PB + 8;           // elements per shared row: 16 bytes more than the row, no bank met twice
 
 template <int N> struct Shape {
@@ -31,7 +32,8 @@ template <int N> struct Shape {
   // in bfloat16 elements: two buffers of C, B, x; three parts of the scores, of the state, of the weighted x
   static constexpr int C0 = 0, B0 = C0 + 2 * Q * NP, X0 = B0 + 2 * Q * NP, M0 = X0 + 2 * Q * XP, S0 = M0 + 3 * Q * MP,
                        W0 = S0 + 3 * N * XP, END = W0 + 3 * Q * XP;
-  static constexpr int BYTES = END * 2 + Q * 8 + 3 * Q * 4;      // and cum (64-bit), dt, e^cum, the rows' weights in the state
+  // and two buffers of cum (64-bit), dt, e^cum, the rows' weights in the state, the state's decay over a chunk
+  static constexpr int BYTES = END * 2 + 2 * (Q * 8 + 3 * Q * 4) + 2 * 4;
 };
 
 __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -83,8 +85,8 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
   extern __shared__ __align__(16) __nv_bfloat16 sm[];
   // [Q] each.  The sums of the a_t are 64-bit: with decays of e^-1 a row their 32-bit sum is 64 times as large as the
   // differences between neighbouring rows that matter, and their error would be ten times that of the row-by-row walk
-  double* cum = reinterpret_cast<double*>(sm + T::END);
-  float *dts = reinterpret_cast<float*>(cum + Q), *ecum = dts + Q, *weight = ecum + Q;
+  double* cum2 = reinterpret_cast<double*>(sm + T::END);
+  float *dts2 = reinterpret_cast<float*>(cum2 + 2 * Q), *ecum2 = dts2 + 2 * Q, *weight2 = ecum2 + 2 * Q, *decay2 = weight2 + 2 * Q;
   pdl_trigger();
   const int h = blockIdx.y, s = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row0 = cu_rows[s], n_rows = cu_rows[s + 1] - row0;      // the step's tables: written before its first kernel
@@ -97,21 +99,21 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
 
   auto load = [&](int c) {      // rows past the segment's end are zeros
     const int buf = c & 1;
-    for (int i = threadIdx.x; i < Q * (N / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < Q * (N / 8); i += WORKERS) {
       const int r = i / (N / 8), k = (i % (N / 8)) * 8;
       const bool valid = c * Q + r < n_rows;
       const __nv_bfloat16* src = xbc + (size_t)(row0 + (valid ? c * Q + r : 0)) * xbc_ld;
       copy16(sm + T::C0 + (buf * Q + r) * NP + k, src + c_col + k, valid);
       copy16(sm + T::B0 + (buf * Q + r) * NP + k, src + b_col + k, valid);
     }
-    for (int i = threadIdx.x; i < Q * (PB / 8); i += THREADS) {
+    for (int i = threadIdx.x; i < Q * (PB / 8); i += WORKERS) {
       const int r = i / (PB / 8), k = (i % (PB / 8)) * 8;
       const bool valid = c * Q + r < n_rows;
       copy16(sm + T::X0 + (buf * Q + r) * XP + k, xbc + (size_t)(row0 + (valid ? c * Q + r : 0)) * xbc_ld + x_col + k, valid);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // the first warp's raw step sizes of a chunk, rows 2 lane and 2 lane + 1
+  // the ninth warp's raw step sizes of a chunk, rows 2 lane and 2 lane + 1
   float raw[2];
   auto load_raw = [&](int c) {
 #pragma unroll
@@ -120,8 +122,48 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
       raw[i] = r < n_rows ? to_f32(proj[(size_t)(row0 + r) * proj_ld + dt_off + h]) : 0.f;
     }
   };
+  // the ninth warp: a chunk's step sizes, decays and weights, from the raw values that it holds
+  auto scalars = [&](int c) {
+    double* cum = cum2 + (c & 1) * Q;
+    float *dts = dts2 + (c & 1) * Q, *ecum = ecum2 + (c & 1) * Q, *weight = weight2 + (c & 1) * Q;
+    float dt[2];
+    double a[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float z = raw[i] + bias;
+      dt[i] = c * Q + 2 * lane + i < n_rows ? (z > 20.f ? z : log1pf(expf(z))) : 0.f;
+      a[i] = (double)neg_a * (double)dt[i];
+    }
+    double up = a[0] + a[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, up, o);
+      if (lane >= o) up += v;
+    }
+    const double last = __shfl_sync(0xffffffffu, up, 31), before = __shfl_up_sync(0xffffffffu, up, 1);
+    const double cs[2] = {(lane ? before : 0.0) + a[0], up};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      cum[2 * lane + i] = cs[i];
+      dts[2 * lane + i] = dt[i];
+      ecum[2 * lane + i] = expf((float)cs[i]);
+      weight[2 * lane + i] = expf((float)(last - cs[i])) * dt[i];
+    }
+    if (lane == 0) decay2[c & 1] = expm1f((float)last);      // (see ssm_scan_kernel: decays close to 1)
+  };
+  if (warp == WORKERS / 32) {
+    load_raw(0);
+    scalars(0);
+    if (n_chunks > 1) load_raw(1);
+    for (int c = 0; c < n_chunks; ++c) {      // the two meetings of every chunk, see below
+      __syncthreads();
+      if (c + 1 < n_chunks) scalars(c + 1);
+      if (c + 2 < n_chunks) load_raw(c + 2);
+      __syncthreads();
+    }
+    return;
+  }
   load(0);
-  if (warp == 0) load_raw(0);
 
   // the state: rows n0 .. n0 + 15 of N, columns p0 .. p0 + 8 S_TILES - 1 of the block's 32, as accumulators (c0, c1: row
   // g, columns 2 t4 and 2 t4 + 1; c2, c3: row g + 8).  In memory a column's N values lie side by side.
@@ -133,45 +175,22 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[j][e] = sp[(size_t)(p0 + 8 * j + 2 * t4 + (e & 1)) * N + n0 + g + 8 * (e >> 1)];
 
-  const int t0 = 16 * (warp & 3), half = warp >> 2;      // this warp's 16 rows of the chunk; which half of the columns
+  // this warp's 16 rows of the chunk and which half of the columns: early rows have little below the diagonal, so that the two
+  // warps of a quarter of the SM (w and w + 4) get an early and a late piece
+  const int half = warp >> 2, t0 = 16 * (half ? 3 - (warp & 3) : warp & 3);
   for (int c = 0; c < n_chunks; ++c) {
     const __nv_bfloat16 *sC = sm + T::C0 + (c & 1) * Q * NP, *sB = sm + T::B0 + (c & 1) * Q * NP, *sX = sm + T::X0 + (c & 1) * Q * XP;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();      // the chunk's rows are there; everyone is done with the chunk before
+    __syncthreads();      // the chunk's rows and scalars are there; everyone is done with the chunk before
     if (c + 1 < n_chunks) load(c + 1);
+    const double* cum = cum2 + (c & 1) * Q;
+    const float *dts = dts2 + (c & 1) * Q, *ecum = ecum2 + (c & 1) * Q, *weight = weight2 + (c & 1) * Q;
     // the state in three parts, [part][n][p]
 #pragma unroll
     for (int j = 0; j < S_TILES; ++j)
 #pragma unroll
       for (int hi = 0; hi < 2; ++hi)
         store_parts(sm + T::S0 + (n0 + g + 8 * hi) * XP + p0 + 8 * j + 2 * t4, N * XP, S[j][2 * hi], S[j][2 * hi + 1]);
-    if (warp == 0) {
-      float dt[2];
-      double a[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const float z = raw[i] + bias;
-        dt[i] = c * Q + 2 * lane + i < n_rows ? (z > 20.f ? z : log1pf(expf(z))) : 0.f;
-        a[i] = (double)neg_a * (double)dt[i];
-      }
-      double up = a[0] + a[1];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, up, o);
-        if (lane >= o) up += v;
-      }
-      const double last = __shfl_sync(0xffffffffu, up, 31), before = __shfl_up_sync(0xffffffffu, up, 1);
-      const double cs[2] = {(lane ? before : 0.0) + a[0], up};
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        cum[2 * lane + i] = cs[i];
-        dts[2 * lane + i] = dt[i];
-        ecum[2 * lane + i] = expf((float)cs[i]);
-        weight[2 * lane + i] = expf((float)(last - cs[i])) * dt[i];
-      }
-      if (c + 1 < n_chunks) load_raw(c + 1);
-    }
-    __syncthreads();
     // ---- scores C B^T of 16 rows and 32 columns, with their decays and step sizes, into [part][t][s]; 0 above the diagonal
     {
       float acc[4][4];
@@ -205,11 +224,12 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
       }
     }
     // ---- x weighted for the state, into [part][s][p]
-    for (int i = threadIdx.x; i < Q * PB / 2; i += THREADS) {
+    for (int i = threadIdx.x; i < Q * PB / 2; i += WORKERS) {
       const int r = i / (PB / 2), p = (i % (PB / 2)) * 2;
       const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sX + r * XP + p));
       store_parts(sm + T::W0 + r * XP + p, Q * XP, weight[r] * x.x, weight[r] * x.y);
     }
+    __syncthreads();      // the parts of the scores, of the state and of the weighted x are there
     // ---- y of 16 rows and 16 columns: first C S from the state before the chunk, then its decay
     float yv[2][4], first[2][4], rest[2][4];
     auto zero = [&]() {
@@ -239,8 +259,7 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
         for (int e = 0; e < 4; ++e) yv[j][e] = (first[j][e] + rest[j][e]) * (e < 2 ? e0 : e1);
     }
     zero();
-    const float decay_m1 = expm1f((float)cum[Q - 1]);      // (see ssm_scan_kernel: decays close to 1)
-    __syncthreads();
+    const float decay_m1 = decay2[c & 1];
     // ---- ... then the chunk's own rows, up to the diagonal
     for (int k = 0; k <= t0; k += 16) {
       uint32_t a[4], b[4];
