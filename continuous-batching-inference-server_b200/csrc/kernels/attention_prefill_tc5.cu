@@ -169,6 +169,37 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// Two 32-bit values an instruction, each with its own rounding; the larger of three; 2^x as the special-function unit gives it
+// (exp2f spends three more instructions on results below 2^-126, which are nothing beside a row's largest, 2^-8 at least).
+// With these a thread's 64 scores take some 250 instructions instead of 520.  Together with the exchange of halves at the end (see
+// there): a prompt of 2,048, 16 heads of 128, 44 -> 36 us; 512 rows behind 512 21.5 -> 17.4; 128 rows 8.9 -> 7.5.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // The 128 softmax threads (warps 2..5) meet at a barrier of their own.
 __device__ __forceinline__ void softmax_warps_meet() {
   __syncwarp();
@@ -177,7 +208,8 @@ __device__ __forceinline__ void softmax_warps_meet() {
 
 // grid: row tiles of the longest segment x heads x segments from seg0 on, in one dimension, times two: the two
 // blocks of a cluster share a row tile, the first takes the first half of its key tiles and the second the rest,
-// and at the end the second hands its sum, reference and output to the first through distributed shared memory.
+// and at the end each hands sum, reference and one half of the head dims to the other through distributed shared memory
+// and finishes the other half.
 // The row tile with the most keys decides how long the kernel runs, and its chain of tiles is halved this way.
 template <int HD, bool BIAS, bool EXT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 2)
@@ -471,15 +503,17 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (i < lo || i >= hi) v[i] = -INFINITY;
         }
       }
-      // four independent chains: a single one would be 64 dependent instructions
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+      // four independent chains, two values an instruction: a single one would be 64 dependent instructions
+      float mx0 = v[0], mx1 = v[1], mx2 = v[2], mx3 = v[3];
 #pragma unroll
-      for (int i = 0; i < BN; i += 4) {
-        mx0 = fmaxf(mx0, v[i]);
-        mx1 = fmaxf(mx1, v[i + 1]);
-        mx2 = fmaxf(mx2, v[i + 2]);
-        mx3 = fmaxf(mx3, v[i + 3]);
+      for (int i = 4; i + 8 <= BN; i += 8) {
+        mx0 = max3(mx0, v[i], v[i + 1]);
+        mx1 = max3(mx1, v[i + 2], v[i + 3]);
+        mx2 = max3(mx2, v[i + 4], v[i + 5]);
+        mx3 = max3(mx3, v[i + 6], v[i + 7]);
       }
+      mx0 = max3(mx0, v[BN - 4], v[BN - 3]);
+      mx1 = max3(mx1, v[BN - 2], v[BN - 1]);
       const float m_tile = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * (BIAS || EXT ? 1.f : scale_log2e);
       // this tile's buffer of P was read by the products of the tile before the last
       if (j > 1 && !bar_wait(&pv_done[j & 1], ((j - 2) >> 1) & 1)) { atomicExch(error, 16); ok = false; TC5_STOP }
@@ -503,23 +537,28 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       if (raise) m = m_tile;
       const float ref = m == -INFINITY ? 0.f : m;   // a row with no key in range yet: every P is exp2(-inf) = 0
       // P = exp2(S * scale - m) in bfloat16 into shared memory (rows of 64 keys, 128-byte swizzle), and its sum
-      float psum = 0.f, psum1 = 0.f;
+      const unsigned long long scale2 = pack2(scale_log2e, scale_log2e), ref2 = pack2(-ref, -ref);
+      unsigned long long psum = 0;
       unsigned char* prow = sP + (j & 1) * P_BYTES + r * 128;
 #pragma unroll
       for (int q8 = 0; q8 < 8; ++q8) {
         unsigned pk[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float e0 = exp2f(BIAS || EXT ? v[q8 * 8 + 2 * i] - ref : fmaf(v[q8 * 8 + 2 * i], scale_log2e, -ref)),
-                      e1 = exp2f(BIAS || EXT ? v[q8 * 8 + 2 * i + 1] - ref : fmaf(v[q8 * 8 + 2 * i + 1], scale_log2e, -ref));
-          psum += e0;
-          psum1 += e1;
+          const unsigned long long x = pack2(v[q8 * 8 + 2 * i], v[q8 * 8 + 2 * i + 1]);
+          float e0, e1;
+          unpack2(BIAS || EXT ? add2(x, ref2) : fma2(x, scale2, ref2), e0, e1);
+          e0 = ex2(e0);
+          e1 = ex2(e1);
+          psum = add2(psum, pack2(e0, e1));
           __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
           pk[i] = *reinterpret_cast<unsigned*>(&b2);
         }
         *reinterpret_cast<uint4*>(prow + ((q8 ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);   // swizzled
       }
-      l += psum + psum1;
+      float psum0, psum1;
+      unpack2(psum, psum0, psum1);
+      l += psum0 + psum1;
       if (j0 + BN > kend && r < BN && j0 + r >= kend && !(EXT && first_no + j < n_kept)) {
         // the last tile: values of keys past the end are whatever the page held; P is zero there, but zero
         // times a NaN left by an earlier owner of the page would still be NaN: this thread clears key row r
@@ -540,25 +579,28 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (ok && n_tiles > 1 && !bar_wait(&pv_done[n_tiles & 1], ((n_tiles - 2) >> 1) & 1)) { atomicExch(error, 16); ok = false; }
     if (ok && n_tiles > 0 && !bar_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1)) { atomicExch(error, 16); ok = false; }
   }
-  // ---- the second block's part goes to the first ------------------------------------------------------------
-  // In the first block's shared memory, where its keys and values were: O as [head dim / 4][row][4] floats (64 KB,
-  // 16 bytes per thread and store, no bank conflicts on either side), then reference and sum per row.
+  // ---- the two blocks' parts meet ------------------------------------------------------------------------------
+  // Each block finishes one half of the head dims: it gets the other block's sums of that half in its shared memory, where its
+  // keys and values were, as [dim / 4][row][4] floats (32 KB, 16 bytes per thread and store, no bank conflicts on either side),
+  // then reference and sum per row.
+  constexpr int HALF = HD / 2;
   const bool softmax_warp = warp >= 2 && warp < 6;
   float* xo = reinterpret_cast<float*>(sK);
-  float* xml = reinterpret_cast<float*>(sK + HD * BM * 4);   // [2][BM], after O (which ends inside P's second buffer)
+  float* xml = reinterpret_cast<float*>(sK + HALF * BM * 4);   // [2][BM], after the sums
+  if (softmax_warp) ok = __all_sync(0xffffffffu, ok);      // (a wait that ran out: the warp stays together)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // the first block's products are done with that memory
-  if (softmax_warp && rank == 1) {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both blocks' products are done with that memory
+  if (softmax_warp) {
     unsigned remote_o, remote_ml;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote_o) : "r"(s32(xo)));
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote_ml) : "r"(s32(xml)));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_o) : "r"(s32(xo)), "r"(rank ^ 1u));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_ml) : "r"(s32(xml)), "r"(rank ^ 1u));
     const bool have = ok && n_tiles > 0;
     if (have) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD; c0 += 32) {
+      for (int c0 = 0; c0 < HALF; c0 += 32) {
         float o[32];
-        tmem_ld32(tmem_o + lane_addr + c0, o);
+        tmem_ld32(tmem_o + lane_addr + (rank ^ 1u) * HALF + c0, o);
 #pragma unroll
         for (int i = 0; i < 32; i += 4)
           asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
@@ -568,58 +610,73 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)(r * 4)), "f"(have ? m : -INFINITY) : "memory");
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)((BM + r) * 4)), "f"(have ? l : 0.f) : "memory");
+    if (!have) m = -INFINITY, l = 0.f;
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // it has arrived
-  if (softmax_warp && rank == 0) {
-    if (ok) {
-      // O = O0 * 2^(m0 - m) + O1 * 2^(m1 - m) with m the larger reference, the sums alike; then O / sum
-      const float m1 = xml[r], l1 = xml[BM + r];
-      const float mm = fmaxf(m, m1);
-      const float f0 = m == -INFINITY ? 0.f : exp2f(m - mm), f1 = (m1 == -INFINITY || l1 == 0.f) ? 0.f : exp2f(m1 - mm);
-      // with the keys cut into chunks the sum stays unnormalised (relative to the reference mm): the merge kernel divides
-      float inv = n_chunks > 1 ? 1.f : 1.f / (l * f0 + l1 * f1);
-      if (sinks && n_chunks == 1) {      // the sink joins the denominator only: with the larger of the two as the reference
-        const float sk = sinks[h] * 1.4426950408889634f, ms = fmaxf(mm, sk), keep = exp2f(mm - ms);
-        inv = keep / fmaf(l * f0 + l1 * f1, keep, exp2f(sk - ms));
-      }
-      const float g0 = f0 * inv, g1 = f1 * inv;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      __nv_bfloat16* dst = out + (size_t)(r_begin + tile * BM + r) * out_ld + h * HD;
-      float* pdst = n_chunks > 1 ? partial + (((size_t)(r_begin + tile * BM + r - row0) * n_head + h) * n_chunks + chunk) * (HD + 4)
-                                 : nullptr;
-      if (pdst && r < rows_here) *reinterpret_cast<float2*>(pdst + HD) = make_float2(mm, l * f0 + l1 * f1);
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // they have arrived
+  if (softmax_warp && ok) {
+    // O = O0 * 2^(m0 - m) + O1 * 2^(m1 - m) with m the larger reference, the sums alike; then O / sum (0: the first block's)
+    const float m_other = xml[r], l_other = xml[BM + r];
+    const float m0 = rank ? m_other : m, l0 = rank ? l_other : l, m1 = rank ? m : m_other, l1 = rank ? l : l_other;
+    const float mm = fmaxf(m0, m1);
+    const float f0 = m0 == -INFINITY ? 0.f : exp2f(m0 - mm), f1 = (m1 == -INFINITY || l1 == 0.f) ? 0.f : exp2f(m1 - mm);
+    // with the keys cut into chunks the sum stays unnormalised (relative to the reference mm): the merge kernel divides
+    float inv = n_chunks > 1 ? 1.f : 1.f / (l0 * f0 + l1 * f1);
+    if (sinks && n_chunks == 1) {      // the sink joins the denominator only: with the larger of the two as the reference
+      const float sk = sinks[h] * 1.4426950408889634f, ms = fmaxf(mm, sk), keep = exp2f(mm - ms);
+      inv = keep / fmaf(l0 * f0 + l1 * f1, keep, exp2f(sk - ms));
+    }
+    const float g0 = f0 * inv, g1 = f1 * inv;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float* pdst = n_chunks > 1 ? partial + (((size_t)(r_begin + tile * BM + r - row0) * n_head + h) * n_chunks + chunk) * (HD + 4)
+                               : nullptr;
+    if (pdst && rank == 0 && r < rows_here) *reinterpret_cast<float2*>(pdst + HD) = make_float2(mm, l0 * f0 + l1 * f1);
+    // A row's bfloat16 results as plain stores of its thread would be 32 rows' partly written lines an instruction: the warp
+    // puts its 32 rows where P was (16-byte pieces, swizzled) and writes them out as whole pieces of rows.
+    constexpr int PIECES = HALF / 8;
+    unsigned char* mine = sP + quarter * (32 * HALF * 2);
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD; c0 += 32) {
-        float o[32];
-        tmem_ld32(tmem_o + lane_addr + c0, o);
-        if (r < rows_here) {
+    for (int c0 = 0; c0 < HALF; c0 += 32) {
+      float o[32];
+      tmem_ld32(tmem_o + lane_addr + rank * HALF + c0, o);
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            float4 o1 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (f1 != 0.f) o1 = *reinterpret_cast<const float4*>(xo + (((c0 + i) >> 2) * BM + r) * 4);
-            o[i] = (f0 != 0.f ? o[i] * g0 : 0.f) + o1.x * g1;
-            o[i + 1] = (f0 != 0.f ? o[i + 1] * g0 : 0.f) + o1.y * g1;
-            o[i + 2] = (f0 != 0.f ? o[i + 2] * g0 : 0.f) + o1.z * g1;
-            o[i + 3] = (f0 != 0.f ? o[i + 3] * g0 : 0.f) + o1.w * g1;
-          }
-          if (pdst) {
+      for (int i = 0; i < 32; i += 4) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if ((rank ? f0 : f1) != 0.f) x = *reinterpret_cast<const float4*>(xo + (((c0 + i) >> 2) * BM + r) * 4);
+        const float other[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int i = 0; i < 32; i += 4)
-              *reinterpret_cast<float4*>(pdst + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-            continue;
-          }
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 q4;
-            __nv_bfloat162 a = __floats2bfloat162_rn(o[i], o[i + 1]), b = __floats2bfloat162_rn(o[i + 2], o[i + 3]);
-            __nv_bfloat162 c = __floats2bfloat162_rn(o[i + 4], o[i + 5]), d = __floats2bfloat162_rn(o[i + 6], o[i + 7]);
-            q4.x = *reinterpret_cast<unsigned*>(&a);
-            q4.y = *reinterpret_cast<unsigned*>(&b);
-            q4.z = *reinterpret_cast<unsigned*>(&c);
-            q4.w = *reinterpret_cast<unsigned*>(&d);
-            *reinterpret_cast<uint4*>(dst + c0 + i) = q4;
-          }
+        for (int e = 0; e < 4; ++e) {
+          const float own = (rank ? f1 : f0) != 0.f ? o[i + e] : 0.f;
+          o[i + e] = fmaf(rank ? own : other[e], g1, (rank ? other[e] : own) * g0);
         }
+      }
+      if (pdst) {
+        if (r < rows_here)
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(pdst + rank * HALF + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        uint4 q4;
+        __nv_bfloat162 a = __floats2bfloat162_rn(o[i], o[i + 1]), b = __floats2bfloat162_rn(o[i + 2], o[i + 3]);
+        __nv_bfloat162 c = __floats2bfloat162_rn(o[i + 4], o[i + 5]), d = __floats2bfloat162_rn(o[i + 6], o[i + 7]);
+        q4.x = *reinterpret_cast<unsigned*>(&a);
+        q4.y = *reinterpret_cast<unsigned*>(&b);
+        q4.z = *reinterpret_cast<unsigned*>(&c);
+        q4.w = *reinterpret_cast<unsigned*>(&d);
+        *reinterpret_cast<uint4*>(mine + lane * (HALF * 2) + ((((c0 + i) >> 3) ^ (lane & (PIECES - 1))) << 4)) = q4;
+      }
+    }
+    if (!pdst) {
+      __syncwarp();
+      __nv_bfloat16* dst = out + (size_t)(r_begin + tile * BM + quarter * 32) * out_ld + h * HD + rank * HALF;
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const int rr = (lane + i * 32) / PIECES, piece = lane % PIECES;
+        if (quarter * 32 + rr < rows_here)
+          *reinterpret_cast<uint4*>(dst + (size_t)rr * out_ld + piece * 8) =
+              *reinterpret_cast<const uint4*>(mine + rr * (HALF * 2) + ((piece ^ (rr & (PIECES - 1))) << 4));
       }
     }
   }
