@@ -198,45 +198,69 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 // With 16-byte aligned rows (STAGES > 0) up to STAGES pieces are on their way at once, the weights' since
 // before the wait for the kernel ahead: piece by piece, each a trip to L2 with nothing else to do, the products of a
 // 256-wide model's decode step took 6.7 us on average; 5.2 so, 4.8 with the blocks spread evenly (common.cuh).
-constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4, FR_STAGE_BYTES = 32 * FR_PITCH * (int)sizeof(float);
+// A walk is bound by its loads from shared memory (two of 16 bytes for four multiply-adds, all of a block's through one SM), so
+// where N is small a block takes 8 or 4 columns instead of 16 and the same loads are spread over two or four times the SMs.  16 rows of 256 columns,
+// K = 1,024: 9.4 us with 16 columns a block and a walk without the next loads on their way, 6.9 now; 768 columns, K = 256: 3.4 and 3.1; one
+// row 3.2 and 2.6.
+constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4;
+constexpr int fr_stage_bytes(int cols) { return (16 + cols) * FR_PITCH * (int)sizeof(float); }
+// Sixteen k at a time, the next sixteen's loads on their way meanwhile: a block has few warps to hide a load's trip behind.
 __device__ __forceinline__ float few_rows_walk(const float* a, const float* w, int kc, float acc) {
-  int k = 0;
-#pragma unroll 8
-  for (; k + 4 <= kc; k += 4) {
-    const float4 av = *reinterpret_cast<const float4*>(a + k), wv = *reinterpret_cast<const float4*>(w + k);
-    acc = fmaf(av.x, wv.x, acc);
-    acc = fmaf(av.y, wv.y, acc);
-    acc = fmaf(av.z, wv.z, acc);
-    acc = fmaf(av.w, wv.w, acc);
+  float4 av[2][4], wv[2][4];
+  auto load = [&](float4 (&x)[4], float4 (&y)[4], int k) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[i] = *reinterpret_cast<const float4*>(a + k + 4 * i);
+      y[i] = *reinterpret_cast<const float4*>(w + k + 4 * i);
+    }
+  };
+  auto add = [&](const float4 (&x)[4], const float4 (&y)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc = fmaf(x[i].x, y[i].x, acc);
+      acc = fmaf(x[i].y, y[i].y, acc);
+      acc = fmaf(x[i].z, y[i].z, acc);
+      acc = fmaf(x[i].w, y[i].w, acc);
+    }
+  };
+  const int n = kc >> 4;
+  if (n > 0) load(av[0], wv[0], 0);
+  int i = 0;
+  for (; i + 1 < n; i += 2) {
+    load(av[1], wv[1], 16 * (i + 1));
+    add(av[0], wv[0]);
+    if (i + 2 < n) load(av[0], wv[0], 16 * (i + 2));
+    add(av[1], wv[1]);
   }
-  for (; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
+  if (i < n) add(av[0], wv[0]);
+  for (int k = 16 * n; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
   return acc;
 }
-template <int STAGES>
-__global__ void __launch_bounds__(256)
+template <int STAGES, int COLS>
+__global__ void __launch_bounds__(16 * COLS)
 linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                            int M, int N, int K, int act, int lda, int ldc) {
-  extern __shared__ __align__(16) float fr_smem[];      // [stages][2][16][FR_PITCH]: A's piece, W's piece
+  extern __shared__ __align__(16) float fr_smem[];      // [stages][16 + COLS][FR_PITCH]: A's piece, W's piece
   pdl_trigger();
   const int tid = threadIdx.x;
-  const int m = tid & 15, c = tid >> 4, n0 = blockIdx.x * 16, n = n0 + c;
+  const int m = tid & 15, c = tid >> 4, n0 = blockIdx.x * COLS, n = n0 + c;
   float acc = 0.f;
   if constexpr (STAGES > 0) {
     const int n_p = (K + FR_KC - 1) / FR_KC, stages = min(n_p, STAGES);
-    auto a_of = [&](int p) { return fr_smem + (size_t)(p % stages) * 32 * FR_PITCH; };
-    auto load = [&](int p, const float* src, int ld, int rows, float* dst) {      // 16 rows of 256: rows past the end are zeros
-      for (int i = tid; i < 16 * (FR_KC / 4); i += 256) {
+    auto a_of = [&](int p) { return fr_smem + (size_t)(p % stages) * (16 + COLS) * FR_PITCH; };
+    auto load = [&](int p, const float* src, int ld, int n_rows, int rows, float* dst) {      // n_rows of 256: rows past the end are zeros
+      for (int i = tid; i < n_rows * (FR_KC / 4); i += 16 * COLS) {
         const int r = i / (FR_KC / 4), k = (i % (FR_KC / 4)) * 4;
         const bool valid = r < rows && p * FR_KC + k < K;
         cp_async16_f32(dst + r * FR_PITCH + k, valid ? src + (size_t)r * ld + p * FR_KC + k : src, valid);
       }
     };
     const float* w0 = W + (size_t)n0 * K;
-    for (int p = 0; p < stages; ++p) load(p, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
+    for (int p = 0; p < stages; ++p) load(p, w0, K, COLS, N - n0, a_of(p) + 16 * FR_PITCH);
     const float b = bias && n < N ? bias[n] : 0.f;
     pdl_wait();  // A comes from the kernel before
     for (int p = 0; p < STAGES; ++p) {
-      if (p < stages) load(p, A, lda, M, a_of(p));
+      if (p < stages) load(p, A, lda, 16, M, a_of(p));
       cp_async_commit();
     }
     for (int p = 0; p < n_p; ++p) {
@@ -246,8 +270,8 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
       acc = few_rows_walk(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
       if (p + stages < n_p) {
         __syncthreads();
-        load(p + stages, w0, K, N - n0, a_of(p) + 16 * FR_PITCH);
-        load(p + stages, A, lda, M, a_of(p));
+        load(p + stages, w0, K, COLS, N - n0, a_of(p) + 16 * FR_PITCH);
+        load(p + stages, A, lda, 16, M, a_of(p));
       }
       cp_async_commit();
     }
@@ -324,12 +348,16 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
     // as long a ring as lets all of an SM's blocks (up to the six that one stage allows) run side by side: 16 rows, K = 2,048, four
     // stages -> this rule: N = 6,144 61 us -> 46, 50,257 442 -> 307; N = 2,304 with one stage 24, with two 21
     const int ring = per_sm <= 1 ? 4 : (per_sm <= 3 ? 2 : 1), stages = !aligned ? 1 : (pieces < ring ? pieces : ring);
-    auto kern = !aligned ? linear_f32_few_rows_kernel<0> : (ring == 4 ? linear_f32_few_rows_kernel<4>
-                         : (ring == 2 ? linear_f32_few_rows_kernel<2> : linear_f32_few_rows_kernel<1>));
+    // 8 or 4 columns a block while that gives an SM no second block
+    const int cols = !aligned || N > 8 * 148 ? 16 : (N > 4 * 148 ? 8 : 4);
+    auto kern = !aligned ? linear_f32_few_rows_kernel<0, 16> : (cols == 8 ? linear_f32_few_rows_kernel<4, 8>
+                         : (cols == 4 ? linear_f32_few_rows_kernel<4, 4> : (ring == 4 ? linear_f32_few_rows_kernel<4, 16>
+                         : (ring == 2 ? linear_f32_few_rows_kernel<2, 16> : linear_f32_few_rows_kernel<1, 16>))));
     size_t smem;
-    cudaError_t e = spread_evenly(kern, (N + 15) / 16, (size_t)stages * FR_STAGE_BYTES, &smem);
+    const int blocks = (N + cols - 1) / cols;
+    cudaError_t e = spread_evenly(kern, blocks, (size_t)stages * fr_stage_bytes(cols), &smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)launch_pdl(kern, dim3((N + 15) / 16), dim3(256), smem, st, A, W, bias, C, M, N, K, act, lda, ldc);
+    return (int)launch_pdl(kern, dim3(blocks), dim3(16 * cols), smem, st, A, W, bias, C, M, N, K, act, lda, ldc);
   }
   dim3 grid((N + 63) / 64, (M + 15) / 16);
   return (int)launch_pdl(linear_f32_kernel<16, 64, 16, 1, 4>, grid, dim3(256), 0, st, A, W, bias, C, M, N, K, w_is_nk,
