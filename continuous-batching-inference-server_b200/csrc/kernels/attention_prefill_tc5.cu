@@ -52,8 +52,15 @@ constexpr int Q_HALF_BYTES = BM * 128;         // 128 rows of 128 bytes: 64 head
 constexpr int KV_HALF_BYTES = BN * 128;        // 64 keys of 128 bytes: 64 head dims
 constexpr int P_BYTES = BM * 128;              // 128 rows of 64 keys
 constexpr int STAGES = 2;
-// Q, keys (one stage), values (STAGES), P (two buffers), barriers; HD: the head size, 64 or 128
-constexpr int smem_bytes(int HD) { return (HD / 64) * (Q_HALF_BYTES + (1 + STAGES) * KV_HALF_BYTES) + 2 * P_BYTES + 128; }
+// Two blocks an SM leave 113 KB each.  At head size 128 that is two stages of keys and one buffer of P: with one stage of keys a
+// tile took as long as its keys' way, 1.1 us in a block of its own (128 rows behind 3,968 keys: 41.4 us, 38.6 so); the
+// products of the tile before have mostly read P by the time it is written.  At head size 64 there is room for two of both
+// (1,023 rows of 25 heads 19.8 us, 20.2 with one buffer of P).
+__host__ __device__ constexpr int p_buffers(int HD) { return HD == 64 ? 2 : 1; }
+// Q, keys and values (STAGES each), P, barriers; HD: the head size, 64 or 128
+constexpr int smem_bytes(int HD) {
+  return (HD / 64) * (Q_HALF_BYTES + 2 * STAGES * KV_HALF_BYTES) + p_buffers(HD) * P_BYTES + 128;
+}
 constexpr int TABLE = BM + BN;                  // entries of the distance bias's table (191 in use)
 constexpr float RAISE_BY = 8.f;                // the reference is raised when a tile's maximum exceeds it by 2^8
 constexpr int THREADS = 224;                   // warp 0: Q and keys, warp 1: MMA + tensor memory, warps 2..5: softmax, warp 6: values
@@ -219,20 +226,20 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                          int n_head, int n_kv_head, int ps, float scale_log2e, int window, int n_chunks, int chunk_keys,
                          float* partial, int row0, int* error, const float* __restrict__ sinks,
                          const float* __restrict__ slopes, const float* __restrict__ rates, int v_heads, float cap, int keep) {
-  constexpr int HALVES = HD / 64, Q_BYTES = HALVES * Q_HALF_BYTES, KV_BYTES = HALVES * KV_HALF_BYTES;
+  constexpr int PBUF = p_buffers(HD), HALVES = HD / 64, Q_BYTES = HALVES * Q_HALF_BYTES, KV_BYTES = HALVES * KV_HALF_BYTES;
   extern __shared__ __align__(1024) unsigned char base[];   // no byte to spare for rounding the address up: checked below
   unsigned char* sQ = base;                                   // 2 halves of the head dim
-  unsigned char* sK = sQ + Q_BYTES;                           // one tile: Q K^T runs two tiles ahead, so the next keys have time
-  unsigned char* sV = sK + KV_BYTES;                          // STAGES tiles
-  unsigned char* sP = sV + STAGES * KV_BYTES;                 // two buffers of 128 rows of 64 keys: P V of a tile runs beside the next softmax
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(sP + 2 * P_BYTES);
+  unsigned char* sK = sQ + Q_BYTES;                           // STAGES tiles
+  unsigned char* sV = sK + STAGES * KV_BYTES;                 // STAGES tiles
+  unsigned char* sP = sV + STAGES * KV_BYTES;                 // PBUF buffers of 128 rows of 64 keys
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(sP + PBUF * P_BYTES);
   // keys and values have barriers of their own: a stage of keys is free as soon as Q K^T has read it, long before
   // the values of the same tile are, so the keys of tile j+2 are on their way while tile j is still being worked on
   unsigned long long *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7,
-                     *s_full = bars + 9, *p_ready = bars + 11, *pv_done = bars + 13;   // k_full/k_empty: [0] only; p_ready, pv_done: [2], tiles in turn
+                     *s_full = bars + 9, *p_ready = bars + 11, *pv_done = bars + 13;   // [2] each but q_full: tiles in turn
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* table = reinterpret_cast<float*>(sP + 2 * P_BYTES + 128);      // BIAS: entry e holds the bias (log2 units) of distance pos0 - j0 - (BN - 1) + e
+  float* table = reinterpret_cast<float*>(sP + PBUF * P_BYTES + 128);      // BIAS: entry e holds the bias (log2 units) of distance pos0 - j0 - (BN - 1) + e
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // late row tiles have the most keys to walk: blocks are numbered so that those of ALL heads and segments come
@@ -290,7 +297,7 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int* bt = block_table + (size_t)seg * max_blocks;
 
   // keys and values of rows that no copy will fill must be finite: P is zero there, and 0 * NaN is NaN
-  for (int i = threadIdx.x; i < (1 + STAGES) * KV_BYTES / 16; i += THREADS)
+  for (int i = threadIdx.x; i < 2 * STAGES * KV_BYTES / 16; i += THREADS)
     reinterpret_cast<uint4*>(sK)[i] = make_uint4(0, 0, 0, 0);
 
   if (threadIdx.x == 0) {
@@ -344,7 +351,7 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int piece = min(ps, BN), pieces_per_tile = BN / piece, piece_shift = 31 - __clz(piece);
     // copies tile j's keys (kv = 0) or values (kv = 1) into their stage; false when the block has given up
     auto load = [&](int j, int kv, int page) -> bool {
-      const int s = kv ? j % STAGES : 0, kt = tile_at(j);   // the keys have one stage
+      const int s = j % STAGES, kt = tile_at(j);
       const int p0 = lane * piece, j0 = kt * BN + p0;
       // runs wholly before the window may lie in pages already given back: they are not read
       const bool mine = lane < pieces_per_tile && ((j0 < kend && j0 + piece > kbegin) || (EXT && j0 < kept_upto));
@@ -355,7 +362,7 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       unsigned long long* full = kv ? &v_full[s] : &k_full[s];
       int stop = 0;
       if (lane == 0) {
-        if (kv ? (j >= STAGES && !bar_wait(&v_empty[s], ((j / STAGES) - 1) & 1)) : (j >= 1 && !bar_wait(&k_empty[0], (j - 1) & 1))) {
+        if (j >= STAGES && !bar_wait(kv ? &v_empty[s] : &k_empty[s], ((j / STAGES) - 1) & 1)) {
           *abort_flag = 1;
           atomicExch(error, 11);
         }
@@ -397,14 +404,15 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       bool ok = bar_wait(q_full, 0);
       if (!ok) { *abort_flag = 2; atomicExch(error, 12); }
       auto issue_qk = [&](int j) -> bool {
-        if (!bar_wait(&k_full[0], j & 1)) { *abort_flag = 3; atomicExch(error, 13); return false; }
+        const int s = j % STAGES;
+        if (!bar_wait(&k_full[s], (j / STAGES) & 1)) { *abort_flag = 3; atomicExch(error, 13); return false; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {   // eight steps of 16 along the head dim, four in each 64-wide half
           mma(tmem_s + (j & 1) * BN, dq + (unsigned)(((kk / 4) * Q_HALF_BYTES + (kk % 4) * 32) >> 4),
-              dk + (unsigned)(((kk / 4) * KV_HALF_BYTES + (kk % 4) * 32) >> 4), idesc(false, BN), kk > 0 ? 1u : 0u);
+              dk + (unsigned)((s * KV_BYTES + (kk / 4) * KV_HALF_BYTES + (kk % 4) * 32) >> 4), idesc(false, BN), kk > 0 ? 1u : 0u);
         }
-        commit(&k_empty[0]);   // the keys' stage is free again when these products have read it
+        commit(&k_empty[s]);   // the keys' stage is free again when these products have read it
         commit(&s_full[j & 1]);
         return true;
       };
@@ -422,7 +430,7 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // head dim KV_HALF_BYTES on
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
-          mma(tmem_o, dp + (unsigned)(((j & 1) * P_BYTES + kk * 32) >> 4), dv + (unsigned)((s * KV_BYTES + kk * 2048) >> 4), idesc(true, HD),
+          mma(tmem_o, dp + (unsigned)(((j % PBUF) * P_BYTES + kk * 32) >> 4), dv + (unsigned)((s * KV_BYTES + kk * 2048) >> 4), idesc(true, HD),
               (j > 0 || kk > 0) ? 1u : 0u);
         }
         commit(&v_empty[s]);   // the values' stage is free again when these products have read it
@@ -515,12 +523,9 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       mx0 = max3(mx0, v[BN - 4], v[BN - 3]);
       mx1 = max3(mx1, v[BN - 2], v[BN - 1]);
       const float m_tile = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * (BIAS || EXT ? 1.f : scale_log2e);
-      // this tile's buffer of P was read by the products of the tile before the last
-      if (j > 1 && !bar_wait(&pv_done[j & 1], ((j - 2) >> 1) & 1)) { atomicExch(error, 16); ok = false; TC5_STOP }
       const bool raise = m_tile > m + RAISE_BY || (m == -INFINITY && m_tile > m);
       if (j > 0 && __any_sync(0xffffffffu, raise)) {
-        // rescale the row of O in tensor memory; rows that keep their reference multiply by 1.  Only here does the
-        // softmax wait for the products of the tile before, which write O.
+        // rescale the row of O in tensor memory, which the products of the tile before write; rows that keep their reference multiply by 1
         if (!bar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1)) { atomicExch(error, 16); ok = false; TC5_STOP }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float f = raise ? exp2f(m - m_tile) : 1.f;
@@ -539,10 +544,9 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       // P = exp2(S * scale - m) in bfloat16 into shared memory (rows of 64 keys, 128-byte swizzle), and its sum
       const unsigned long long scale2 = pack2(scale_log2e, scale_log2e), ref2 = pack2(-ref, -ref);
       unsigned long long psum = 0;
-      unsigned char* prow = sP + (j & 1) * P_BYTES + r * 128;
+      unsigned pk[8][4];
 #pragma unroll
       for (int q8 = 0; q8 < 8; ++q8) {
-        unsigned pk[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const unsigned long long x = pack2(v[q8 * 8 + 2 * i], v[q8 * 8 + 2 * i + 1]);
@@ -552,10 +556,15 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           e1 = ex2(e1);
           psum = add2(psum, pack2(e0, e1));
           __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
-          pk[i] = *reinterpret_cast<unsigned*>(&b2);
+          pk[q8][i] = *reinterpret_cast<unsigned*>(&b2);
         }
-        *reinterpret_cast<uint4*>(prow + ((q8 ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);   // swizzled
       }
+      // the products that read this buffer of P last have done so by the time this tile's exponentials are there
+      if (j >= PBUF && !bar_wait(&pv_done[(j - PBUF) & 1], ((j - PBUF) >> 1) & 1)) { atomicExch(error, 16); ok = false; TC5_STOP }
+      unsigned char* prow = sP + (j % PBUF) * P_BYTES + r * 128;
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8)
+        *reinterpret_cast<uint4*>(prow + ((q8 ^ (r & 7)) << 4)) = make_uint4(pk[q8][0], pk[q8][1], pk[q8][2], pk[q8][3]);   // swizzled
       float psum0, psum1;
       unpack2(psum, psum0, psum1);
       l += psum0 + psum1;
