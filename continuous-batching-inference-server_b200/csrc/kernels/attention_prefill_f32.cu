@@ -248,8 +248,9 @@ paged_prefill_f32_kernel(const float* q, int q_ld, const float* kc, const float*
 // 32 bits, are cut once per block into shared memory while the next tile is on its way, and P is cut in registers, where the
 // scores' accumulators already lie as the next product's operand.  Bound by the tensor cores' legacy path (192 products a
 // warp and tile at head size 32) beside the exponentials and the cutting.
-// 512 rows behind 8,192 keys, 8 heads of 32, with the merge of the chunks: 131 us, where the first kernel took 173 and its
-// multiply-adds alone take 59; behind 30,000 keys 457 and 643; head size 64 behind 4,096 keys 141 and 169; one tile of 13 rows 4.8 and 5.2.
+// 512 rows behind 8,192 keys, 8 heads of 32, with the merge of the chunks: 126 us, where the first kernel took 173 and its
+// multiply-adds alone take 59; behind 30,000 keys 453 and 643; head size 64 behind 4,096 keys 137 and 169; one tile of 13 rows 4.9 and 5.2.
+// Three blocks an SM at head size 32: four, of 128 registers a thread, gain 3 % behind 8,192 keys and lose a third where there are few tiles.
 // Against 64 bits it is no further off than sums of 32-bit products one by one.
 //
 // A value that is not finite has parts that are no numbers: a tile with one, or with one of 10^18 and more (a row tile, for q),
@@ -472,17 +473,22 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
     float corr[2];
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
-      const int p = pos0 + wr + g + 8 * hi, lo = edge ? max(kbegin, first_seen(p, window)) : 0, up = edge ? min(kend, p + 1) : j0 + M_BN;
+      if (edge) {      // the keys this row sees: [lo, up) of the tile; a tile that all rows see whole is not compared (131 -> 126 us)
+        const int p = pos0 + wr + g + 8 * hi, lo = max(kbegin, first_seen(p, window)) - j0, up = min(kend, p + 1) - j0;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int j = 8 * n + 2 * t4 + e;
+            s[n][2 * hi + e] = j >= lo && j < up ? s[n][2 * hi + e] * scale : -INFINITY;
+          }
+      } else {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) s[n][2 * hi] *= scale, s[n][2 * hi + 1] *= scale;
+      }
       float mx = -INFINITY;
 #pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 8 * n + 2 * t4 + e;
-          float& v = s[n][2 * hi + e];
-          v = (j >= lo && j < up) ? v * scale : -INFINITY;
-          mx = fmaxf(mx, v);
-        }
+      for (int n = 0; n < 8; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * hi], s[n][2 * hi + 1]));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       const float m_new = fmaxf(m[hi], mx);
