@@ -225,7 +225,7 @@ def _plain(ctx, mixer, qkv, cache, view, out, nd, T, hd, ps, k_pages, v_pages, k
                                             mixer.window, chunks, partial)
             if ctx.n_segments > nd:
                 # (three blocks fit on an SM at head size 32, two at 48 to 128; pieces for five to eight times as many, so that the
-                # last ones leave few SMs idle: 2,048 rows of 8 heads of 32 110 us with half as many, 91 so; 48 to 96 the same either way)
+                # last ones leave few SMs idle: 2,048 rows of 8 heads of 32 80 us with half as many, 71 so; 48 to 96 the same either way)
                 chunks, partial = _key_chunks(ctx, mixer.n_head, nd, T, hd, blocks_per_sm=16)
                 ops.paged_prefill_f32(qkv, k_pages, v_pages, view.block_table, ctx.cu_rows, ctx.seg_start, out, nd,
                                       ctx.n_segments - nd, ctx.max_seg_rows, mixer.n_head, mixer.n_kv_head, hd, ps,
