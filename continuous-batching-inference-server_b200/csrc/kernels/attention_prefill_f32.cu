@@ -306,7 +306,7 @@ __device__ __forceinline__ void mma_parts(float (&first)[4], float (&rest)[4], c
 
 // The grid and the arguments of paged_prefill_f32_kernel.
 template <int HD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, HD <= 16 ? 4 : (HD <= 32 ? 3 : 2))
 paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const float* vc, const int* block_table, int max_blocks,
                              const int* cu_rows, const int* seg_start, float* out, int out_ld, int seg0, int n_head,
                              int n_kv_head, int ps, float scale, int window, int n_chunks, int chunk_keys, float* partial, int row0) {
@@ -543,6 +543,14 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
       for (int n = 0; n < ND; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[n][e] *= corr[e >> 1];
+      // a key that a row does not see has weight 0 there, but 0 times a value that is not finite would be no number
+      int lo[2], up[2];
+#pragma unroll
+      for (int hi = 0; hi < 2; ++hi) {
+        const int p = pos0 + wr + g + 8 * hi;
+        lo[hi] = max(kbegin, first_seen(p, window)) - j0;
+        up[hi] = min(kend, p + 1) - j0;
+      }
 #pragma unroll
       for (int kn = 0; kn < 8; ++kn)
 #pragma unroll 1
@@ -550,14 +558,16 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
             const float p0 = __shfl_sync(0xffffffffu, s[kn][b], (lane & ~3) + src), p1 = __shfl_sync(0xffffffffu, s[kn][2 + b], (lane & ~3) + src);
-            const float* vr = fV + (8 * kn + 2 * src + b) * HD + 2 * t4;
+            const int j = 8 * kn + 2 * src + b;
+            const bool in0 = j >= lo[0] && j < up[0], in1 = j >= lo[1] && j < up[1];
+            const float* vr = fV + j * HD + 2 * t4;
 #pragma unroll
             for (int n = 0; n < ND; ++n) {
               const float2 v = *reinterpret_cast<const float2*>(vr + 8 * n);
-              o[n][0] = fmaf(p0, v.x, o[n][0]);
-              o[n][1] = fmaf(p0, v.y, o[n][1]);
-              o[n][2] = fmaf(p1, v.x, o[n][2]);
-              o[n][3] = fmaf(p1, v.y, o[n][3]);
+              o[n][0] = fmaf(p0, in0 ? v.x : 0.f, o[n][0]);
+              o[n][1] = fmaf(p0, in0 ? v.y : 0.f, o[n][1]);
+              o[n][2] = fmaf(p1, in1 ? v.x : 0.f, o[n][2]);
+              o[n][3] = fmaf(p1, in1 ? v.y : 0.f, o[n][3]);
             }
           }
       __syncthreads();      // everyone has read the copy

@@ -6,34 +6,39 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def run(q, k, v, n_head, hd, ps, window=0):
-    """The rows of one sequence (all of its positions), pages in a mixed order -> (tiled form, general form), [T, heads * hd]."""
+def run(q, k, v, n_head, hd, ps, window=0, chunks=(1, 0)):
+    """The last rows of one sequence (all of it, or a portion behind a context), pages in a mixed order -> (tiled form, general
+    form), [rows, heads * hd]."""
     from cbis_b200.kernels import ops
-    T = q.shape[0]
+    T, rows = k.shape[0], q.shape[0]
     n_kv_head, n_pages = k.shape[1], -(-T // ps)
     bt = torch.randperm(n_pages, generator=torch.Generator().manual_seed(T)).to(torch.int32)
     kc, vc = (torch.zeros(n_pages, n_kv_head, ps, hd, device="cuda") for _ in range(2))
     pos = torch.arange(T)
-    for cache, rows in ((kc, k), (vc, v)):
-        cache[bt[pos // ps].long().cuda(), :, (pos % ps).cuda()] = rows.cuda()
-    cu = torch.tensor([0, T], dtype=torch.int32, device="cuda")
-    start = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for cache, values in ((kc, k), (vc, v)):
+        cache[bt[pos // ps].long().cuda(), :, (pos % ps).cuda()] = values.cuda()
+    cu = torch.tensor([0, rows], dtype=torch.int32, device="cuda")
+    start = torch.tensor([T - rows], dtype=torch.int32, device="cuda")
+    pos = pos[T - rows:].to(torch.int32).cuda()
     bt = bt[None].contiguous().cuda()
-    qd = q.reshape(T, -1).cuda()
+    qd = q.reshape(rows, -1).cuda()
     tiled, general = torch.empty_like(qd), torch.empty_like(qd)
-    ops.paged_prefill_f32(qd, kc, vc, bt, cu, start, tiled, 0, 1, T, n_head, n_kv_head, hd, ps, hd ** -0.5, window)
-    ops.paged_attention_generic(qd, kc, vc, bt, torch.zeros(T, dtype=torch.int32, device="cuda"),
-                                pos.to(torch.int32).cuda(), general, n_head, n_kv_head, hd, ps, hd ** -0.5, window)
+    partial = torch.full((rows * n_head * chunks[0] * (hd + 4),), float("nan"), device="cuda") if chunks[0] > 1 else None
+    ops.paged_prefill_f32(qd, kc, vc, bt, cu, start, tiled, 0, 1, rows, n_head, n_kv_head, hd, ps, hd ** -0.5, window, chunks, partial,
+                          pos, 0, rows)
+    ops.paged_attention_generic(qd, kc, vc, bt, torch.zeros(rows, dtype=torch.int32, device="cuda"), pos, general, n_head,
+                                n_kv_head, hd, ps, hd ** -0.5, window)
     return tiled.cpu(), general.cpu()
 
 
-def exact(q, k, v, hd):
-    T, H = q.shape[:2]
-    per = H // k.shape[1]
+def exact(q, k, v, hd, window=0):
+    rows, H = q.shape[:2]
+    T, per = k.shape[0], H // k.shape[1]
     k, v = (x.double().repeat_interleave(per, 1).permute(1, 0, 2) for x in (k, v))
     s = torch.matmul(q.double().permute(1, 0, 2), k.transpose(1, 2)) * hd ** -0.5
-    s.masked_fill_(torch.ones(T, T, dtype=torch.bool).triu(1), float("-inf"))
-    return torch.matmul(torch.softmax(s, -1), v).permute(1, 0, 2).reshape(T, -1)
+    back = torch.arange(T - rows, T)[:, None] - torch.arange(T)[None]
+    s.masked_fill_((back < 0) | ((back >= window) if window else False), float("-inf"))
+    return torch.matmul(torch.softmax(s, -1), v).permute(1, 0, 2).reshape(rows, -1)
 
 
 @pytest.mark.parametrize("T", [1, 63, 64, 65, 700])
@@ -50,18 +55,18 @@ def test_error_against_64_bits(T, hd, n_head, n_kv_head, size):
     assert e_tiled <= 1.2 * e_general + 3e-8, (e_tiled, e_general)
 
 
-@pytest.mark.parametrize("hd", [16, 32, 64])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("hd", [16, 32, 48, 64])
 @pytest.mark.parametrize("what, value", [("k", float("-inf")), ("k", 1e30), ("v", float("inf")), ("v", -3e38), ("v", float("nan")),
                                          ("q", 1e20), ("q", float("inf"))])
-def test_values_that_cannot_be_cut(hd, what, value):
-    """One such value, at position 70: rows before its tile and rows from its own on are those of the general form (rows
-    between share a tile with it, where 0 times it may be no number in either tiled form)."""
+def test_values_that_cannot_be_cut(hd, what, value, window):
+    """One such value, at position 70, in a tile with rows that see it and rows that do not (those before it, with a window those
+    far behind it): all rows are those of the general form, which walks only the keys that a row sees."""
     T, at = 200, 70
     g = torch.Generator().manual_seed(hd)
     q, k, v = (torch.randn(T, 2, hd, generator=g) for _ in range(3))
     q[:, :, 3] = q[:, :, 3].abs() + 0.1
     {"q": q, "k": k, "v": v}[what][at, 1, 3] = value
-    tiled, general = run(q, k, v, 2, hd, 16)
-    for rows in (slice(0, 64), slice(at, T)):
-        assert torch.equal(torch.isfinite(tiled[rows]), torch.isfinite(general[rows]))
-        assert torch.allclose(tiled[rows], general[rows], rtol=3e-6, atol=3e-6, equal_nan=True)
+    tiled, general = run(q, k, v, 2, hd, 16, window)
+    assert torch.equal(torch.isfinite(tiled), torch.isfinite(general))
+    assert torch.allclose(tiled, general, rtol=3e-6, atol=3e-6, equal_nan=True)
