@@ -17,6 +17,7 @@
 // and leaves its unnormalised sum, maximum and denominator in scratch memory, and a second kernel merges the
 // chunks of every row.
 #include "attention_merge.cuh"
+#include "packed.cuh"
 
 namespace cbis {
 
@@ -255,7 +256,11 @@ paged_prefill_f32_kernel(const float* q, int q_ld, const float* kc, const float*
 //
 // A value that is not finite has parts that are no numbers: a tile with one, or with one of 10^18 and more (a row tile, for q),
 // is worked out value by value from the 32-bit copies instead, and the next tile is fetched only then.
+// Values are cut at 2^60 times their size, and a tile's sums go back to theirs: as they are, values below 2^-109 or so would lose
+// their third parts (1e-35: 3e-6 off instead of 2e-7), scaled no part of any 32-bit value is too small for bfloat16, and the sum of
+// 64 weights of at most 1 times less than 10^18 stays below the largest number.
 constexpr int M_BM = 64, M_BN = 64;
+constexpr float V_UP = 1152921504606846976.f, V_DOWN = 1.f / V_UP;      // 2^60
 template <int HD> struct F32MmaTile {
   static constexpr int PITCH = HD + 8;                                    // bfloat16 elements of a part's row: no bank met twice
   static constexpr int STAGE = 2 * M_BN * HD;                             // floats of a tile's keys and values as they come
@@ -415,8 +420,13 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
 #pragma unroll
     for (int n = 0; n < 2 * COPIES; ++n) {
       const int i = tid + n * 128, rr = i / (HD / 4), c = (i % (HD / 4)) * 4;      // keys, then values: rows 64 on
-      const float4 v = *reinterpret_cast<const float4*>(fK + rr * HD + c);
+      float4 v = *reinterpret_cast<const float4*>(fK + rr * HD + c);
       good = good && can_cut(v.x) && can_cut(v.y) && can_cut(v.z) && can_cut(v.w);
+      if (n >= COPIES) {
+        const unsigned long long up = pack2(V_UP, V_UP);
+        unpack2(mul2(pack2(v.x, v.y), up), v.x, v.y);
+        unpack2(mul2(pack2(v.z, v.w), up), v.z, v.w);
+      }
       unsigned lo[3], hi[3];
       cut3(v.x, v.y, lo);
       cut3(v.z, v.w, hi);
@@ -534,10 +544,14 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
           mma_parts(first[nd + 1], rest[nd + 1], pa, b[0][2], b[0][3], b[1][2], b[1][3], b[2][2], b[2][3]);
         }
       }
+      const unsigned long long down = pack2(V_DOWN, V_DOWN), corr2[2] = {pack2(corr[0], corr[0]), pack2(corr[1], corr[1])};
 #pragma unroll
       for (int n = 0; n < ND; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[n][e] = fmaf(o[n][e], corr[e >> 1], first[n][e] + rest[n][e]);
+        for (int hi = 0; hi < 2; ++hi) {
+          const unsigned long long sum = add2(pack2(first[n][2 * hi], first[n][2 * hi + 1]), pack2(rest[n][2 * hi], rest[n][2 * hi + 1]));
+          unpack2(fma2(pack2(o[n][2 * hi], o[n][2 * hi + 1]), corr2[hi], mul2(sum, down)), o[n][2 * hi], o[n][2 * hi + 1]);
+        }
     } else {
 #pragma unroll
       for (int n = 0; n < ND; ++n)

@@ -39,6 +39,7 @@
 // Every wait on an mbarrier is bounded; when a limit runs out the block sets *error, stops, frees its
 // tensor memory and returns (its output rows are then invalid, and the host raises).
 #include "attention_merge.cuh"
+#include "packed.cuh"
 
 #include <cuda.h>
 #include <math.h>
@@ -180,22 +181,6 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const float* v) {
 // (exp2f spends three more instructions on results below 2^-126, which are nothing beside a row's largest, 2^-8 at least).
 // With these a thread's 64 scores take some 250 instructions instead of 520.  Together with the exchange of halves at the end (see
 // there): a prompt of 2,048, 16 heads of 128, 44 -> 36 us; 512 rows behind 512 21.5 -> 17.4; 128 rows 8.9 -> 7.5.
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));

@@ -55,6 +55,20 @@ def test_error_against_64_bits(T, hd, n_head, n_kv_head, size):
     assert e_tiled <= 1.2 * e_general + 3e-8, (e_tiled, e_general)
 
 
+@pytest.mark.parametrize("hd", [16, 32, 48, 64])
+@pytest.mark.parametrize("size", [1e-30, 1e-35, 1e-38, 1e-41])
+def test_small_values(hd, size):
+    """Values down to the smallest that 32 bits hold, whose third parts as they are would be too small for bfloat16: the bound of
+    the test above, with half a step of such numbers (7e-46) for every rounding of an output."""
+    g = torch.Generator().manual_seed(hd)
+    q, k, v = (torch.randn(150, 2, hd, generator=g) for _ in range(3))
+    v = (v + 2.0) * size
+    tiled, general = run(q, k, v, 2, hd, 16)
+    ref = exact(q, k, v, hd)
+    e_tiled, e_general = ((x.double() - ref).norm() / ref.norm() for x in (tiled, general))
+    assert e_tiled <= 1.2 * e_general + 3e-8 + 7e-46 / size, (e_tiled, e_general)
+
+
 @pytest.mark.parametrize("window", [0, 40])
 @pytest.mark.parametrize("hd", [16, 32, 48, 64])
 @pytest.mark.parametrize("what, value", [("k", float("-inf")), ("k", 1e30), ("v", float("inf")), ("v", -3e38), ("v", float("nan")),
