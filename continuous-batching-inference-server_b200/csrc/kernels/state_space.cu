@@ -34,38 +34,14 @@ __device__ __forceinline__ void store_v(TT* p, const float* v) {
   else from_f32(*p, v[0]);
 }
 
-// grid (ceil(C / (128 V)), S, ceil(max rows of a segment / kConvRows)), 128 threads of V neighbouring channels each.
-// u = in[r, c0 + c]; out[r, c] = act(bias[c] + sum_j w[c, j] * u[t - (K-1) + j]), j = 0..K-1.
-// state[slot][j][c], j = 0..K-2, holds the input K-1-j rows before the segment's first row.
-// What bounds it are instructions, not bytes: eight rows' sums wait in registers and are activated together, so that the
-// choice among the activations is made once for 8 V values.  With the choice beside every value a warp jumped through
+// R rows at a time of a segment's rows first .. last - 1, V neighbouring channels; src, dst: the segment's first row.
+// What bounds it are instructions, not bytes: the rows' sums wait in registers and are activated together, so that the
+// choice among the activations is made once for R V values.  With the choice beside every value a warp jumped through
 // tens of kilobytes of code: 25.5 us for 1,500 rows of 6,144 channels of 4 taps, 21.5 now.  The rows after are on their
 // way while these are worked on.
-// R rows at a time: eight, or one where segments have a row or two (decoding: eight would activate seven sums that are not there,
-// 3.0 us against 1.4 for 6,144 channels; with the choice beside every value 2.3).
 template <typename TT, int K, int V, int R>
-__global__ void __launch_bounds__(128)
-causal_conv_act_kernel(const TT* in, int in_ld, int c0, const float* __restrict__ w, const float* __restrict__ bias,
-                       float* state, long long slot_stride, const int* seg_slot, const int* cu_rows, TT* out,
-                       int out_ld, int C, int act, int update_state) {
-  pdl_trigger();
-  const int c = (blockIdx.x * 128 + threadIdx.x) * V;
-  const int s = blockIdx.y;
-  const int first = blockIdx.z * kConvRows;
-  float wk[V][K], b[V];      // weights: no kernel before this one writes them
-#pragma unroll
-  for (int e = 0; e < V; ++e) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) wk[e][j] = c < C ? w[(size_t)(c + e) * K + j] : 0.f;
-    b[e] = bias && c < C ? bias[c + e] : 0.f;
-  }
-  const int row0 = cu_rows[s], n = cu_rows[s + 1] - row0;      // the step's tables: written before its first kernel
-  float* st = state + (long long)seg_slot[s] * slot_stride + c;
-  pdl_wait();
-  if (c >= C || first >= n) return;
-  const int last = min(n, first + kConvRows);
-  const TT* src = in + (size_t)row0 * in_ld + c0 + c;
-  TT* dst = out + (size_t)row0 * out_ld + c;
+__device__ __forceinline__ void conv_rows(const TT* src, int in_ld, const float (&wk)[V][K], const float (&b)[V], float* st, TT* dst,
+                                          int out_ld, int C, int act, int update_state, int first, int last) {
   // win: the K - 1 inputs before the next row, then R rows' own
   float win[K - 1 + R][V], next[R][V];
 #pragma unroll
@@ -136,13 +112,53 @@ causal_conv_act_kernel(const TT* in, int in_ld, int c0, const float* __restrict_
   }
 }
 
-template <typename TT, int V, int R>
+// grid (ceil(C / (128 V)), S, ceil(max rows of a segment / kConvRows)), 128 threads of V neighbouring channels each.
+// u = in[r, c0 + c]; out[r, c] = act(bias[c] + sum_j w[c, j] * u[t - (K-1) + j]), j = 0..K-1.
+// state[slot][j][c], j = 0..K-2, holds the input K-1-j rows before the segment's first row.
+// A block takes its segment's rows eight at a time, four where the segment ends with this block, one where it has a row or two (a
+// decoding request, alone or beside a prompt portion): a batch activates all of its sums, also those that are not there.  4 taps,
+// 6,144 channels: one row 1.6 us (in a batch of eight 3.0; with the choice beside every value 2.3), 200 rows of their own beside
+// five 12.8 (26.5; 19.6), 50 segments of six rows 7.8 (9.5; 9.1).
+// ALL_FEW: no segment of the step has more than two rows, and the code for more is left out.
+template <typename TT, int K, int V, bool ALL_FEW>
+__global__ void __launch_bounds__(128)
+causal_conv_act_kernel(const TT* in, int in_ld, int c0, const float* __restrict__ w, const float* __restrict__ bias,
+                       float* state, long long slot_stride, const int* seg_slot, const int* cu_rows, TT* out,
+                       int out_ld, int C, int act, int update_state) {
+  pdl_trigger();
+  const int c = (blockIdx.x * 128 + threadIdx.x) * V;
+  const int s = blockIdx.y;
+  const int first = blockIdx.z * kConvRows;
+  const int row0 = cu_rows[s], n = cu_rows[s + 1] - row0;      // the step's tables: written before its first kernel
+  if (!ALL_FEW && blockIdx.z > 0 && first >= n) {      // (a short segment beside a long one: most of its blocks)
+    pdl_wait();
+    return;
+  }
+  float wk[V][K], b[V];      // weights: no kernel before this one writes them
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) wk[e][j] = c < C ? w[(size_t)(c + e) * K + j] : 0.f;
+    b[e] = bias && c < C ? bias[c + e] : 0.f;
+  }
+  float* st = state + (long long)seg_slot[s] * slot_stride + c;
+  pdl_wait();
+  if (c >= C || first >= n) return;
+  const int last = min(n, first + kConvRows);
+  const TT* src = in + (size_t)row0 * in_ld + c0 + c;
+  TT* dst = out + (size_t)row0 * out_ld + c;
+  if (ALL_FEW || n <= 2) conv_rows<TT, K, V, 1>(src, in_ld, wk, b, st, dst, out_ld, C, act, update_state, first, last);
+  else if (n <= kConvRows) conv_rows<TT, K, V, 4>(src, in_ld, wk, b, st, dst, out_ld, C, act, update_state, first, last);
+  else conv_rows<TT, K, V, 8>(src, in_ld, wk, b, st, dst, out_ld, C, act, update_state, first, last);
+}
+
+template <typename TT, int V, bool ALL_FEW>
 static int launch_conv(int K, dim3 grid, cudaStream_t st, const TT* in, int in_ld, int c0, const float* w, const float* bias,
                        float* state, long long slot_stride, const int* seg_slot, const int* cu_rows, TT* out, int out_ld, int C,
                        int act, int update_state) {
 #define CBIS_CONV(K_)                                                                                                     \
   case K_:                                                                                                                \
-    return (int)launch_pdl(causal_conv_act_kernel<TT, K_, V, R>, grid, dim3(128), 0, st, in, in_ld, c0, w, bias, state,      \
+    return (int)launch_pdl(causal_conv_act_kernel<TT, K_, V, ALL_FEW>, grid, dim3(128), 0, st, in, in_ld, c0, w, bias, state, \
                            slot_stride, seg_slot, cu_rows, out, out_ld, C, act, update_state)
   switch (K) {
     CBIS_CONV(1); CBIS_CONV(2); CBIS_CONV(3); CBIS_CONV(4); CBIS_CONV(5); CBIS_CONV(6); CBIS_CONV(7); CBIS_CONV(8);
@@ -151,26 +167,24 @@ static int launch_conv(int K, dim3 grid, cudaStream_t st, const TT* in, int in_l
   return CBIS_ERR_BAD_SIZE;
 }
 
-// Two channels a thread where every row's pairs are aligned and that still gives every SM a block (100 rows of 6,144 channels of
-// 8 taps, 96 blocks: 10.0 us, with one channel a thread 9.8), else one; one row at a time where no segment has more than two.
+// Two channels a thread where every row's pairs are aligned, the taps are few and the step's rows, most of them in long segments,
+// give blocks of pairs in numbers that run at once (128 registers a thread: four an SM) and leave no SM idle; else one.  4 taps,
+// one channel a thread -> two: 23 rows of their own beside 489 of 6,144 channels 24.3 us -> 19.9, 512 rows 12.1 -> 11.9, 1,500 rows of
+// 2,304 channels 12.2 -> 11.9; but 3 x 200 rows of 2,304 (171 blocks) 9.4 -> 11.0, 1,500 rows of 6,144 (1,128) 21.5 -> 22.7; 8 taps, 512
+// rows of 6,144 10.9 -> 14.3.
 template <typename TT>
-static int launch_conv_for(int K, int n_segments, int max_seg_rows, cudaStream_t st, const TT* in, int in_ld, int c0, const float* w,
-                           const float* bias, float* state, long long slot_stride, const int* seg_slot, const int* cu_rows,
-                           TT* out, int out_ld, int C, int act, int update_state) {
+static int launch_conv_for(int K, int n_segments, int n_rows, int max_seg_rows, cudaStream_t st, const TT* in, int in_ld, int c0,
+                           const float* w, const float* bias, float* state, long long slot_stride, const int* seg_slot,
+                           const int* cu_rows, TT* out, int out_ld, int C, int act, int update_state) {
   const bool few = max_seg_rows <= 2;
   const int row_blocks = (max_seg_rows + kConvRows - 1) / kConvRows;
-  const bool pairs = !few && (long long)((C + 255) / 256) * n_segments * row_blocks >= 148 && C % 2 == 0 && c0 % 2 == 0 && in_ld % 2 == 0 && out_ld % 2 == 0 &&
-                     (((uintptr_t)in | (uintptr_t)out) & (2 * sizeof(TT) - 1)) == 0;
+  const long long in_pairs = (long long)((C + 255) / 256) * ((n_rows + kConvRows - 1) / kConvRows);
+  const bool pairs = max_seg_rows > kConvRows && K <= 4 && in_pairs >= 256 && in_pairs <= 4 * 148 && 2 * n_segments <= n_rows && C % 2 == 0 &&
+                     c0 % 2 == 0 && in_ld % 2 == 0 && out_ld % 2 == 0 && (((uintptr_t)in | (uintptr_t)out) & (2 * sizeof(TT) - 1)) == 0;
   const int per_block = pairs ? 256 : 128;
   const dim3 grid((C + per_block - 1) / per_block, n_segments, row_blocks);
-  if (few)
-    return launch_conv<TT, 1, 1>(K, grid, st, in, in_ld, c0, w, bias, state, slot_stride, seg_slot, cu_rows, out, out_ld, C, act,
-                                 update_state);
-  if (pairs)
-    return launch_conv<TT, 2, 8>(K, grid, st, in, in_ld, c0, w, bias, state, slot_stride, seg_slot, cu_rows, out, out_ld, C, act,
-                              update_state);
-  return launch_conv<TT, 1, 8>(K, grid, st, in, in_ld, c0, w, bias, state, slot_stride, seg_slot, cu_rows, out, out_ld, C, act,
-                            update_state);
+  auto launch = few ? launch_conv<TT, 1, true> : (pairs ? launch_conv<TT, 2, false> : launch_conv<TT, 1, false>);
+  return launch(K, grid, st, in, in_ld, c0, w, bias, state, slot_stride, seg_slot, cu_rows, out, out_ld, C, act, update_state);
 }
 
 // grid (ceil(C / 128), S): state[slot][j][c] <- the input K-1-j rows before the row after the segment's last.
@@ -481,15 +495,15 @@ CBIS_EXPORT int cbis_conv_max_taps() { return kMaxTaps; }
 CBIS_EXPORT int cbis_scan_max_state() { return 256; }
 
 // in: [T, in_ld] of the compute type, the convolution's channels at columns c0 .. c0 + C - 1; out: [T, out_ld].
-// w [C, K] and bias [C] 32-bit; state: 32-bit, (K-1) * C floats at `state + slot * slot_stride`.
+// w [C, K] and bias [C] 32-bit; state: 32-bit, (K-1) * C floats at `state + slot * slot_stride`; n_rows: the step's, T.
 CBIS_EXPORT int cbis_conv_rows_per_block() { return kConvRows; }
 
 // `update_state` (max_seg_rows <= cbis_conv_rows_per_block() only): the kernel also leaves the state as
 // cbis_conv_state_update would.
 CBIS_EXPORT int cbis_causal_conv_act(const void* in, int in_ld, int c0, const float* w, const float* bias,
                                      float* state, long long slot_stride, const int* seg_slot, const int* cu_rows,
-                                     void* out, int out_ld, int C, int K, int act, int n_segments, int max_seg_rows,
-                                     int update_state, int dtype, void* stream) {
+                                     void* out, int out_ld, int C, int K, int act, int n_segments, int n_rows,
+                                     int max_seg_rows, int update_state, int dtype, void* stream) {
   if (n_segments <= 0 || max_seg_rows <= 0) return CBIS_OK;
   if (C <= 0 || K < 1 || K > kMaxTaps) return CBIS_ERR_BAD_SIZE;
   if (update_state && max_seg_rows > kConvRows) return CBIS_ERR_BAD_SIZE;
@@ -497,10 +511,10 @@ CBIS_EXPORT int cbis_causal_conv_act(const void* in, int in_ld, int c0, const fl
   if ((max_seg_rows + kConvRows - 1) / kConvRows > 65535) return CBIS_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == CBIS_F32)
-    return launch_conv_for(K, n_segments, max_seg_rows, st, (const float*)in, in_ld, c0, w, bias, state, slot_stride, seg_slot,
+    return launch_conv_for(K, n_segments, n_rows, max_seg_rows, st, (const float*)in, in_ld, c0, w, bias, state, slot_stride, seg_slot,
                            cu_rows, (float*)out, out_ld, C, act, update_state);
   if (dtype == CBIS_BF16)
-    return launch_conv_for(K, n_segments, max_seg_rows, st, (const __nv_bfloat16*)in, in_ld, c0, w, bias, state, slot_stride,
+    return launch_conv_for(K, n_segments, n_rows, max_seg_rows, st, (const __nv_bfloat16*)in, in_ld, c0, w, bias, state, slot_stride,
                            seg_slot, cu_rows, (__nv_bfloat16*)out, out_ld, C, act, update_state);
   return CBIS_ERR_BAD_DTYPE;
 }

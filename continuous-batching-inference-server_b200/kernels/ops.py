@@ -1409,8 +1409,8 @@ def causal_conv_act(x, c0, channels, weight, bias, state, seg_slot, cu_rows, n_s
     st = kernels().cbis_causal_conv_act(_ptr(x), c_int(x.stride(0)), c_int(c0), _ptr(weight), _ptr(bias), _ptr(state),
                                         ctypes.c_longlong(state.stride(0)), _ptr(seg_slot), _ptr(cu_rows), _ptr(out),
                                         c_int(out.stride(0)), c_int(channels), c_int(taps), c_int(ACT[act]),
-                                        c_int(n_segments), c_int(max_seg_rows), c_int(1 if update_state else 0),
-                                        c_int(dtype_code(x.dtype)), _stream())
+                                        c_int(n_segments), c_int(x.shape[0]), c_int(max_seg_rows),
+                                        c_int(1 if update_state else 0), c_int(dtype_code(x.dtype)), _stream())
     _check(st, "causal_conv_act", f"channels={channels} taps={taps} segments={n_segments}")
 
 
