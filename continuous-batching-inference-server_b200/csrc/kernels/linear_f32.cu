@@ -189,9 +189,9 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 }
 
 // Up to 16 rows (decoding) with W stored [N, K]: the tiled kernel above would run N / 64 blocks that walk K in
-// steps of 16 with two barriers each: 62 us for a 16 x 768 x 256 product.  Here a block takes 16 output columns
+// steps of 16 with two barriers each: 62 us for a 16 x 768 x 256 product.  Here a block takes 16, 8 or 4 output columns
 // and a thread owns ONE output (lane m of a half-warp: row m; the half-warp: one column).  K comes in pieces of
-// 256: the block copies the piece of A (16 rows) and of W (16 rows) into shared memory with coalesced 16-byte
+// 256: the block copies the piece of A (16 rows) and of W (its columns) into shared memory with coalesced 16-byte
 // loads, all in flight at once, and every thread then walks its piece from left to right with one fused
 // multiply-add per element: the same order as the tiled kernel, hence the same bits, so that a token decoded
 // alone and the same token inside a prompt portion still agree exactly.
@@ -204,39 +204,53 @@ linear_f32_nk_kernel(const float* A, const float* __restrict__ W, const float* _
 // row 3.2 and 2.6.
 constexpr int FR_KC = 256, FR_PITCH = FR_KC + 4;
 constexpr int fr_stage_bytes(int cols) { return (16 + cols) * FR_PITCH * (int)sizeof(float); }
-// Sixteen k at a time, the next sixteen's loads on their way meanwhile: a block has few warps to hide a load's trip behind.
+// AHEAD: sixteen k at a time, the next sixteen's loads on their way meanwhile, where a block has few warps to hide a load's trip
+// behind; not for pieces under 128, which end before that pays.
+template <bool AHEAD>
 __device__ __forceinline__ float few_rows_walk(const float* a, const float* w, int kc, float acc) {
-  float4 av[2][4], wv[2][4];
-  auto load = [&](float4 (&x)[4], float4 (&y)[4], int k) {
+  int k = 0;
+  if (AHEAD && kc >= 128) {
+    float4 av[2][4], wv[2][4];
+    auto load = [&](float4 (&x)[4], float4 (&y)[4], int k) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      x[i] = *reinterpret_cast<const float4*>(a + k + 4 * i);
-      y[i] = *reinterpret_cast<const float4*>(w + k + 4 * i);
-    }
-  };
-  auto add = [&](const float4 (&x)[4], const float4 (&y)[4]) {
+      for (int i = 0; i < 4; ++i) {
+        x[i] = *reinterpret_cast<const float4*>(a + k + 4 * i);
+        y[i] = *reinterpret_cast<const float4*>(w + k + 4 * i);
+      }
+    };
+    auto add = [&](const float4 (&x)[4], const float4 (&y)[4]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc = fmaf(x[i].x, y[i].x, acc);
-      acc = fmaf(x[i].y, y[i].y, acc);
-      acc = fmaf(x[i].z, y[i].z, acc);
-      acc = fmaf(x[i].w, y[i].w, acc);
+      for (int i = 0; i < 4; ++i) {
+        acc = fmaf(x[i].x, y[i].x, acc);
+        acc = fmaf(x[i].y, y[i].y, acc);
+        acc = fmaf(x[i].z, y[i].z, acc);
+        acc = fmaf(x[i].w, y[i].w, acc);
+      }
+    };
+    const int n = kc >> 4;
+    load(av[0], wv[0], 0);
+    int i = 0;
+    for (; i + 1 < n; i += 2) {
+      load(av[1], wv[1], 16 * (i + 1));
+      add(av[0], wv[0]);
+      if (i + 2 < n) load(av[0], wv[0], 16 * (i + 2));
+      add(av[1], wv[1]);
     }
-  };
-  const int n = kc >> 4;
-  if (n > 0) load(av[0], wv[0], 0);
-  int i = 0;
-  for (; i + 1 < n; i += 2) {
-    load(av[1], wv[1], 16 * (i + 1));
-    add(av[0], wv[0]);
-    if (i + 2 < n) load(av[0], wv[0], 16 * (i + 2));
-    add(av[1], wv[1]);
+    if (i < n) add(av[0], wv[0]);
+    k = 16 * n;
   }
-  if (i < n) add(av[0], wv[0]);
-  for (int k = 16 * n; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
+#pragma unroll 8
+  for (; k + 4 <= kc; k += 4) {
+    const float4 av = *reinterpret_cast<const float4*>(a + k), wv = *reinterpret_cast<const float4*>(w + k);
+    acc = fmaf(av.x, wv.x, acc);
+    acc = fmaf(av.y, wv.y, acc);
+    acc = fmaf(av.z, wv.z, acc);
+    acc = fmaf(av.w, wv.w, acc);
+  }
+  for (; k < kc; ++k) acc = fmaf(a[k], w[k], acc);
   return acc;
 }
-template <int STAGES, int COLS>
+template <int STAGES, int COLS, bool AHEAD>
 __global__ void __launch_bounds__(16 * COLS)
 linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                            int M, int N, int K, int act, int lda, int ldc) {
@@ -267,7 +281,7 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
       cp_async_wait<STAGES - 1>();
       __syncthreads();
       const float* a = a_of(p);
-      acc = few_rows_walk(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
+      acc = few_rows_walk<AHEAD>(a + m * FR_PITCH, a + (16 + c) * FR_PITCH, min(FR_KC, K - p * FR_KC), acc);
       if (p + stages < n_p) {
         __syncthreads();
         load(p + stages, w0, K, COLS, N - n0, a_of(p) + 16 * FR_PITCH);
@@ -286,6 +300,7 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
   pdl_wait();  // A comes from the kernel before
   for (int k0 = 0; k0 < K; k0 += FR_KC) {
     const int kc = min(FR_KC, K - k0);
+#pragma unroll
     for (int i = tid; i < 16 * FR_KC; i += 256) {
       const int r = i / FR_KC, k = i % FR_KC;
       As[r][k] = (k < kc && r < M) ? A[(size_t)r * lda + k0 + k] : 0.f;
@@ -294,7 +309,7 @@ linear_f32_few_rows_kernel(const float* A, const float* __restrict__ W, const fl
     __syncthreads();
     // (a piece shorter than 256 ends in zeros of A and W: adding 0 * 0 changes no bit of the sum... except the sign of
     // a zero sum, so the loop stops at the piece's end)
-    acc = few_rows_walk(As[m], Ws[c], kc, acc);
+    acc = few_rows_walk<AHEAD>(As[m], Ws[c], kc, acc);
     __syncthreads();
   }
   if (m < M && n < N) {
@@ -342,17 +357,24 @@ CBIS_EXPORT int cbis_linear_f32(const float* A, const float* W, const float* bia
     return (int)launch_pdl(linear_f32_kernel<64, 64, 16, 4, 4>, grid, dim3(256), 0, st, A, W, bias, C, M, N, K, w_is_nk,
                            act, lda, ldc);
   }
-  if (w_is_nk) {   // decoding: one thread per output, 16 outputs (rows) x 2 columns per warp, 8 warps per block
+  if (w_is_nk) {   // decoding: one thread per output, 16 outputs (rows) x 2 columns per warp, a warp for every two columns of a block
     const bool aligned = K % 4 == 0 && lda % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
     const int pieces = (K + FR_KC - 1) / FR_KC, per_sm = ((N + 15) / 16 + 147) / 148;
     // as long a ring as lets all of an SM's blocks (up to the six that one stage allows) run side by side: 16 rows, K = 2,048, four
     // stages -> this rule: N = 6,144 61 us -> 46, 50,257 442 -> 307; N = 2,304 with one stage 24, with two 21
     const int ring = per_sm <= 1 ? 4 : (per_sm <= 3 ? 2 : 1), stages = !aligned ? 1 : (pieces < ring ? pieces : ring);
-    // 8 or 4 columns a block while that gives an SM no second block
-    const int cols = !aligned || N > 8 * 148 ? 16 : (N > 4 * 148 ? 8 : 4);
-    auto kern = !aligned ? linear_f32_few_rows_kernel<0, 16> : (cols == 8 ? linear_f32_few_rows_kernel<4, 8>
-                         : (cols == 4 ? linear_f32_few_rows_kernel<4, 4> : (ring == 4 ? linear_f32_few_rows_kernel<4, 16>
-                         : (ring == 2 ? linear_f32_few_rows_kernel<2, 16> : linear_f32_few_rows_kernel<1, 16>))));
+    // 8 or 4 columns a block while that gives an SM no second block, and while the walk is long enough to pay for more blocks: not under
+    // K = 128 (16 rows of 592 columns, K = 64: 2.2 -> 2.7 us), and under 256, but for a row or four, only up to half as many blocks
+    // (16 rows, K = 128: 592 columns in 148 blocks 2.6 -> 2.8)
+    const int most = K < 128 ? 0 : (K < FR_KC && M > 4 ? 74 : 148);
+    const int cols = !aligned || N > 8 * most ? 16 : (N > 4 * most ? 8 : 4);
+    // Loads ahead in the walk take registers: with them three blocks of 16 columns fit on an SM instead of six, and one alone has
+    // warps enough without (16 rows, K = 2,048: N = 1,185 19.0 us without and 19.8 with, 3,072 32.7 and 31.2, 7,200 58.8 and 63.4)
+    const bool ahead = ring == 2 && K >= 3 * FR_KC;
+    auto kern = !aligned ? linear_f32_few_rows_kernel<0, 16, false> : (cols == 8 ? linear_f32_few_rows_kernel<4, 8, true>
+                         : (cols == 4 ? linear_f32_few_rows_kernel<4, 4, true> : (ring == 4 ? linear_f32_few_rows_kernel<4, 16, false>
+                         : (ring == 1 ? linear_f32_few_rows_kernel<1, 16, false> : (ahead ? linear_f32_few_rows_kernel<2, 16, true>
+                         : linear_f32_few_rows_kernel<2, 16, false>)))));
     size_t smem;
     const int blocks = (N + cols - 1) / cols;
     cudaError_t e = spread_evenly(kern, blocks, (size_t)stages * fr_stage_bytes(cols), &smem);

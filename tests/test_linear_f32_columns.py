@@ -6,15 +6,15 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N", [1, 5, 256, 592, 593, 1184, 1185])
-@pytest.mark.parametrize("K", [4, 16, 20, 256, 300, 1044])
+@pytest.mark.parametrize("N", [1, 5, 256, 296, 297, 592, 593, 1184, 1185, 2500])
+@pytest.mark.parametrize("K", [4, 16, 20, 124, 128, 252, 256, 300, 768, 1044])
 def test_few_rows_have_the_bits_of_the_tiled_kernel(N, K):
     from cbis_b200.kernels import ops
     g = torch.Generator().manual_seed(N + K)
     x, w, b = torch.randn(16, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda(), torch.randn(N, generator=g).cuda()
     want = torch.empty(32, N, device="cuda")
     ops.linear_f32(torch.cat([x, x]), w, b, None, want, w_is_nk=True)      # more than 16 rows: tiles
-    for rows in (1, 7, 16):
+    for rows in (1, 4, 5, 7, 16):
         got = torch.full((rows, N), float("nan"), device="cuda")
         ops.linear_f32(x[:rows], w, b, None, got, w_is_nk=True)
         assert torch.equal(got, want[:rows])
