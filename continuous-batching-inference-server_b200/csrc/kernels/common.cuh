@@ -186,6 +186,15 @@ inline cudaError_t spread_evenly(Kern kern, long long blocks, size_t need, size_
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
 }
 
+// Lets a kernel be launched with `smem` bytes of dynamic shared memory (at most 200 KB).  What it holds besides (under 1 KB in every
+// kernel that comes here) counts toward the 48 KB that need no leave: a limit of 48 KB on `smem` alone refused rows of 6,144 entries
+// in two buffers.  One value whatever the size: another thread may be between its call of this and its launch.
+template <typename Kern>
+inline cudaError_t allow_smem(Kern kern, size_t smem) {
+  if (smem <= 47 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+}
+
 // Activations in 32-bit.  GELU, erf form: kernels/elementwise.cu:59-66 of the reference; tanh form: GPT-2's gelu_new;
 // silu(v) = v * sigmoid(v); sigmoid alone is the activation of a gate.
 __device__ __forceinline__ float sigmoid_f32(float v) { return 1.0f / (1.0f + expf(-v)); }

@@ -206,8 +206,8 @@ CBIS_EXPORT int cbis_add_rmsnorm(float* x, const void* delta, int delta_ld, int 
   cudaStream_t st = (cudaStream_t)stream;
 #define CBIS_ARN(TD, TO)                                                                                              \
   do {                                                                                                                \
-    if (smem > 48 * 1024)                                                                                             \
-      cudaFuncSetAttribute(add_rmsnorm_kernel<TD, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+    const cudaError_t e = allow_smem(add_rmsnorm_kernel<TD, TO>, smem);                                               \
+    if (e != cudaSuccess) return (int)e;                                                                              \
     return (int)launch_pdl(add_rmsnorm_kernel<TD, TO>, dim3(n), dim3(threads), smem, st, x, (const TD*)delta, delta_ld, \
                            delta_bias, post_w, post_eps, post_offset, w, eps, offset, (TO*)out, rows, d, delta_scale, \
                            x_scale, stream_w, stream_eps, stream_offset);                                             \

@@ -264,8 +264,8 @@ CBIS_EXPORT int cbis_qk_prepare(void* buf, int ld, int q_off, int q_heads, int k
   cudaStream_t st = (cudaStream_t)stream;
 #define CBIS_QKP(TT)                                                                                                  \
   do {                                                                                                                \
-    if (smem > 48 * 1024)                                                                                             \
-      cudaFuncSetAttribute(qk_prepare_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
+    const cudaError_t e = allow_smem(qk_prepare_kernel<TT>, smem);                                                    \
+    if (e != cudaSuccess) return (int)e;                                                                              \
     return (int)launch_pdl(qk_prepare_kernel<TT>, dim3(rows), dim3(threads), smem, st, (TT*)buf, ld, q_off, q_heads,  \
                            k_off, k_heads, width, q_w, k_w, eps, positions, freqs, dims, v_off, d_v,                  \
                            (const TT*)v_other, v_other_ld, lambda, table);                                            \
