@@ -57,10 +57,11 @@ constexpr int STAGES = 2;
 // tile took as long as its keys' way, 1.1 us in a block of its own (128 rows behind 3,968 keys: 41.4 us, 38.6 so); the
 // products of the tile before have mostly read P by the time it is written.  At head size 64 there is room for two of both
 // (1,023 rows of 25 heads 19.8 us, 20.2 with one buffer of P).
+constexpr int FLAG_BYTES = 144;                // barriers and flags
 __host__ __device__ constexpr int p_buffers(int HD) { return HD == 64 ? 2 : 1; }
 // Q, keys and values (STAGES each), P, barriers; HD: the head size, 64 or 128
 constexpr int smem_bytes(int HD) {
-  return (HD / 64) * (Q_HALF_BYTES + 2 * STAGES * KV_HALF_BYTES) + p_buffers(HD) * P_BYTES + 128;
+  return (HD / 64) * (Q_HALF_BYTES + 2 * STAGES * KV_HALF_BYTES) + p_buffers(HD) * P_BYTES + FLAG_BYTES;
 }
 constexpr int TABLE = BM + BN;                  // entries of the distance bias's table (191 in use)
 constexpr float RAISE_BY = 8.f;                // the reference is raised when a tile's maximum exceeds it by 2^8
@@ -224,7 +225,8 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                      *s_full = bars + 9, *p_ready = bars + 11, *pv_done = bars + 13;   // [2] each but q_full: tiles in turn
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* table = reinterpret_cast<float*>(sP + PBUF * P_BYTES + 128);      // BIAS: entry e holds the bias (log2 units) of distance pos0 - j0 - (BN - 1) + e
+  volatile int* alone_flag = abort_flag + 1;                 // one tile of keys in all (kept here: the loops have no register to spare)
+  float* table = reinterpret_cast<float*>(sP + PBUF * P_BYTES + FLAG_BYTES);      // BIAS: entry e holds the bias (log2 units) of distance pos0 - j0 - (BN - 1) + e
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // late row tiles have the most keys to walk: blocks are numbered so that those of ALL heads and segments come
@@ -281,9 +283,9 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   };
   const int* bt = block_table + (size_t)seg * max_blocks;
 
-  // keys and values of rows that no copy will fill must be finite: P is zero there, and 0 * NaN is NaN
-  for (int i = threadIdx.x; i < 2 * STAGES * KV_BYTES / 16; i += THREADS)
-    reinterpret_cast<uint4*>(sK)[i] = make_uint4(0, 0, 0, 0);
+  // keys and values of rows that no copy will fill must be finite: P is zero there, and 0 * NaN is NaN (only in the stages in use)
+  for (int i = threadIdx.x; i < min(n_tiles, STAGES) * KV_BYTES / 16; i += THREADS)
+    reinterpret_cast<uint4*>(sK)[i] = reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
 
   if (threadIdx.x == 0) {
     bar_init(q_full, 1);
@@ -300,6 +302,7 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     bar_init(&pv_done[0], 1);
     bar_init(&pv_done[1], 1);
     *abort_flag = 0;
+    *alone_flag = n_all == 1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -576,101 +579,137 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   // ---- the two blocks' parts meet ------------------------------------------------------------------------------
   // Each block finishes one half of the head dims: it gets the other block's sums of that half in its shared memory, where its
   // keys and values were, as [dim / 4][row][4] floats (32 KB, 16 bytes per thread and store, no bank conflicts on either side),
-  // then reference and sum per row.
+  // then reference and sum per row.  A single tile of keys is the first block's alone, and so are both halves.
   constexpr int HALF = HD / 2;
   const bool softmax_warp = warp >= 2 && warp < 6;
   float* xo = reinterpret_cast<float*>(sK);
   float* xml = reinterpret_cast<float*>(sK + HALF * BM * 4);   // [2][BM], after the sums
   if (softmax_warp) ok = __all_sync(0xffffffffu, ok);      // (a wait that ran out: the warp stays together)
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both blocks' products are done with that memory
-  if (softmax_warp) {
-    unsigned remote_o, remote_ml;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_o) : "r"(s32(xo)), "r"(rank ^ 1u));
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_ml) : "r"(s32(xml)), "r"(rank ^ 1u));
-    const bool have = ok && n_tiles > 0;
-    if (have) {
+  if (*alone_flag) {      // (both blocks of the cluster alike; 17 rows, 4 heads of 128: 7.5 us with halves exchanged, 5.7 so)
+    if (softmax_warp && ok && rank == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float inv = n_chunks > 1 ? 1.f : 1.f / l;
+      if (sinks && n_chunks == 1) {
+        const float sk = sinks[h] * 1.4426950408889634f, ms = fmaxf(m, sk), keep = exp2f(m - ms);
+        inv = keep / fmaf(l, keep, exp2f(sk - ms));
+      }
+      __nv_bfloat16* dst = out + (size_t)(r_begin + tile * BM + r) * out_ld + h * HD;
+      float* pdst = n_chunks > 1 ? partial + (((size_t)(r_begin + tile * BM + r - row0) * n_head + h) * n_chunks + chunk) * (HD + 4)
+                                 : nullptr;
+      if (pdst && r < rows_here) *reinterpret_cast<float2*>(pdst + HD) = make_float2(m, l);
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD; c0 += 32) {
+        float o[32];
+        tmem_ld32(tmem_o + lane_addr + c0, o);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = m == -INFINITY ? 0.f * inv : fmaf(o[i], inv, 0.f);
+        if (r < rows_here && pdst) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(pdst + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        } else if (r < rows_here) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            const __nv_bfloat162 b[4] = {__floats2bfloat162_rn(o[i], o[i + 1]), __floats2bfloat162_rn(o[i + 2], o[i + 3]),
+                                         __floats2bfloat162_rn(o[i + 4], o[i + 5]), __floats2bfloat162_rn(o[i + 6], o[i + 7])};
+            *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(*reinterpret_cast<const unsigned*>(&b[0]), *reinterpret_cast<const unsigned*>(&b[1]),
+                                                                 *reinterpret_cast<const unsigned*>(&b[2]), *reinterpret_cast<const unsigned*>(&b[3]));
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both blocks' products are done with that memory
+    if (softmax_warp) {
+      unsigned remote_o, remote_ml;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_o) : "r"(s32(xo)), "r"(rank ^ 1u));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_ml) : "r"(s32(xml)), "r"(rank ^ 1u));
+      const bool have = ok && n_tiles > 0;
+      if (have) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+        for (int c0 = 0; c0 < HALF; c0 += 32) {
+          float o[32];
+          tmem_ld32(tmem_o + lane_addr + (rank ^ 1u) * HALF + c0, o);
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                         ::"r"(remote_o + (unsigned)((((c0 + i) >> 2) * BM + r) * 16)), "f"(o[i]), "f"(o[i + 1]), "f"(o[i + 2]), "f"(o[i + 3])
+                         : "memory");
+        }
+      }
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)(r * 4)), "f"(have ? m : -INFINITY) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)((BM + r) * 4)), "f"(have ? l : 0.f) : "memory");
+      if (!have) m = -INFINITY, l = 0.f;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // they have arrived
+    if (softmax_warp && ok) {
+      // O = O0 * 2^(m0 - m) + O1 * 2^(m1 - m) with m the larger reference, the sums alike; then O / sum (0: the first block's)
+      const float m_other = xml[r], l_other = xml[BM + r];
+      const float m0 = rank ? m_other : m, l0 = rank ? l_other : l, m1 = rank ? m : m_other, l1 = rank ? l : l_other;
+      const float mm = fmaxf(m0, m1);
+      const float f0 = m0 == -INFINITY ? 0.f : exp2f(m0 - mm), f1 = (m1 == -INFINITY || l1 == 0.f) ? 0.f : exp2f(m1 - mm);
+      // with the keys cut into chunks the sum stays unnormalised (relative to the reference mm): the merge kernel divides
+      float inv = n_chunks > 1 ? 1.f : 1.f / (l0 * f0 + l1 * f1);
+      if (sinks && n_chunks == 1) {      // the sink joins the denominator only: with the larger of the two as the reference
+        const float sk = sinks[h] * 1.4426950408889634f, ms = fmaxf(mm, sk), keep = exp2f(mm - ms);
+        inv = keep / fmaf(l0 * f0 + l1 * f1, keep, exp2f(sk - ms));
+      }
+      const float g0 = f0 * inv, g1 = f1 * inv;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float* pdst = n_chunks > 1 ? partial + (((size_t)(r_begin + tile * BM + r - row0) * n_head + h) * n_chunks + chunk) * (HD + 4)
+                                 : nullptr;
+      if (pdst && rank == 0 && r < rows_here) *reinterpret_cast<float2*>(pdst + HD) = make_float2(mm, l0 * f0 + l1 * f1);
+      // A row's bfloat16 results as plain stores of its thread would be 32 rows' partly written lines an instruction: the warp
+      // puts its 32 rows where P was (16-byte pieces, swizzled) and writes them out as whole pieces of rows.
+      constexpr int PIECES = HALF / 8;
+      unsigned char* mine = sP + quarter * (32 * HALF * 2);
 #pragma unroll 1
       for (int c0 = 0; c0 < HALF; c0 += 32) {
         float o[32];
-        tmem_ld32(tmem_o + lane_addr + (rank ^ 1u) * HALF + c0, o);
+        tmem_ld32(tmem_o + lane_addr + rank * HALF + c0, o);
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
-                       ::"r"(remote_o + (unsigned)((((c0 + i) >> 2) * BM + r) * 16)), "f"(o[i]), "f"(o[i + 1]), "f"(o[i + 2]), "f"(o[i + 3])
-                       : "memory");
-      }
-    }
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)(r * 4)), "f"(have ? m : -INFINITY) : "memory");
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_ml + (unsigned)((BM + r) * 4)), "f"(have ? l : 0.f) : "memory");
-    if (!have) m = -INFINITY, l = 0.f;
-  }
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // they have arrived
-  if (softmax_warp && ok) {
-    // O = O0 * 2^(m0 - m) + O1 * 2^(m1 - m) with m the larger reference, the sums alike; then O / sum (0: the first block's)
-    const float m_other = xml[r], l_other = xml[BM + r];
-    const float m0 = rank ? m_other : m, l0 = rank ? l_other : l, m1 = rank ? m : m_other, l1 = rank ? l : l_other;
-    const float mm = fmaxf(m0, m1);
-    const float f0 = m0 == -INFINITY ? 0.f : exp2f(m0 - mm), f1 = (m1 == -INFINITY || l1 == 0.f) ? 0.f : exp2f(m1 - mm);
-    // with the keys cut into chunks the sum stays unnormalised (relative to the reference mm): the merge kernel divides
-    float inv = n_chunks > 1 ? 1.f : 1.f / (l0 * f0 + l1 * f1);
-    if (sinks && n_chunks == 1) {      // the sink joins the denominator only: with the larger of the two as the reference
-      const float sk = sinks[h] * 1.4426950408889634f, ms = fmaxf(mm, sk), keep = exp2f(mm - ms);
-      inv = keep / fmaf(l0 * f0 + l1 * f1, keep, exp2f(sk - ms));
-    }
-    const float g0 = f0 * inv, g1 = f1 * inv;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float* pdst = n_chunks > 1 ? partial + (((size_t)(r_begin + tile * BM + r - row0) * n_head + h) * n_chunks + chunk) * (HD + 4)
-                               : nullptr;
-    if (pdst && rank == 0 && r < rows_here) *reinterpret_cast<float2*>(pdst + HD) = make_float2(mm, l0 * f0 + l1 * f1);
-    // A row's bfloat16 results as plain stores of its thread would be 32 rows' partly written lines an instruction: the warp
-    // puts its 32 rows where P was (16-byte pieces, swizzled) and writes them out as whole pieces of rows.
-    constexpr int PIECES = HALF / 8;
-    unsigned char* mine = sP + quarter * (32 * HALF * 2);
-#pragma unroll 1
-    for (int c0 = 0; c0 < HALF; c0 += 32) {
-      float o[32];
-      tmem_ld32(tmem_o + lane_addr + rank * HALF + c0, o);
+        for (int i = 0; i < 32; i += 4) {
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+          if ((rank ? f0 : f1) != 0.f) x = *reinterpret_cast<const float4*>(xo + (((c0 + i) >> 2) * BM + r) * 4);
+          const float other[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if ((rank ? f0 : f1) != 0.f) x = *reinterpret_cast<const float4*>(xo + (((c0 + i) >> 2) * BM + r) * 4);
-        const float other[4] = {x.x, x.y, x.z, x.w};
+          for (int e = 0; e < 4; ++e) {
+            const float own = (rank ? f1 : f0) != 0.f ? o[i + e] : 0.f;
+            o[i + e] = fmaf(rank ? own : other[e], g1, (rank ? other[e] : own) * g0);
+          }
+        }
+        if (pdst) {
+          if (r < rows_here)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float own = (rank ? f1 : f0) != 0.f ? o[i + e] : 0.f;
-          o[i + e] = fmaf(rank ? own : other[e], g1, (rank ? other[e] : own) * g0);
+            for (int i = 0; i < 32; i += 4)
+              *reinterpret_cast<float4*>(pdst + rank * HALF + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+          continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          uint4 q4;
+          __nv_bfloat162 a = __floats2bfloat162_rn(o[i], o[i + 1]), b = __floats2bfloat162_rn(o[i + 2], o[i + 3]);
+          __nv_bfloat162 c = __floats2bfloat162_rn(o[i + 4], o[i + 5]), d = __floats2bfloat162_rn(o[i + 6], o[i + 7]);
+          q4.x = *reinterpret_cast<unsigned*>(&a);
+          q4.y = *reinterpret_cast<unsigned*>(&b);
+          q4.z = *reinterpret_cast<unsigned*>(&c);
+          q4.w = *reinterpret_cast<unsigned*>(&d);
+          *reinterpret_cast<uint4*>(mine + lane * (HALF * 2) + ((((c0 + i) >> 3) ^ (lane & (PIECES - 1))) << 4)) = q4;
         }
       }
-      if (pdst) {
-        if (r < rows_here)
+      if (!pdst) {
+        __syncwarp();
+        __nv_bfloat16* dst = out + (size_t)(r_begin + tile * BM + quarter * 32) * out_ld + h * HD + rank * HALF;
 #pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(pdst + rank * HALF + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-        continue;
-      }
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 q4;
-        __nv_bfloat162 a = __floats2bfloat162_rn(o[i], o[i + 1]), b = __floats2bfloat162_rn(o[i + 2], o[i + 3]);
-        __nv_bfloat162 c = __floats2bfloat162_rn(o[i + 4], o[i + 5]), d = __floats2bfloat162_rn(o[i + 6], o[i + 7]);
-        q4.x = *reinterpret_cast<unsigned*>(&a);
-        q4.y = *reinterpret_cast<unsigned*>(&b);
-        q4.z = *reinterpret_cast<unsigned*>(&c);
-        q4.w = *reinterpret_cast<unsigned*>(&d);
-        *reinterpret_cast<uint4*>(mine + lane * (HALF * 2) + ((((c0 + i) >> 3) ^ (lane & (PIECES - 1))) << 4)) = q4;
-      }
-    }
-    if (!pdst) {
-      __syncwarp();
-      __nv_bfloat16* dst = out + (size_t)(r_begin + tile * BM + quarter * 32) * out_ld + h * HD + rank * HALF;
-#pragma unroll
-      for (int i = 0; i < PIECES; ++i) {
-        const int rr = (lane + i * 32) / PIECES, piece = lane % PIECES;
-        if (quarter * 32 + rr < rows_here)
-          *reinterpret_cast<uint4*>(dst + (size_t)rr * out_ld + piece * 8) =
-              *reinterpret_cast<const uint4*>(mine + rr * (HALF * 2) + ((piece ^ (rr & (PIECES - 1))) << 4));
+        for (int i = 0; i < PIECES; ++i) {
+          const int rr = (lane + i * 32) / PIECES, piece = lane % PIECES;
+          if (quarter * 32 + rr < rows_here)
+            *reinterpret_cast<uint4*>(dst + (size_t)rr * out_ld + piece * 8) =
+                *reinterpret_cast<const uint4*>(mine + rr * (HALF * 2) + ((piece ^ (rr & (PIECES - 1))) << 4));
+        }
       }
     }
   }
