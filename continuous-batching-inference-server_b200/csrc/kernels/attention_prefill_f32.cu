@@ -1,11 +1,12 @@
-// Prefill attention over the paged cache in true 32-bit: the 32-bit path's counterpart of the tiled kernels; head sizes above
-// 64 by multiply-adds (the first kernel), up to 64 as products of parts on the tensor cores (the second).  The reference gives every (row, head) a warp that walks all keys of the prefix one by one, so a
+// Prefill attention over the paged cache of 32-bit values: the 32-bit path's counterpart of the tiled kernels; head sizes above
+// 64 by 32-bit multiply-adds (the first kernel), up to 64 as products of bfloat16 parts on the tensor cores (the second).  The
+// reference gives every (row, head) a warp that walks all keys of the prefix one by one, so a
 // prefill re-reads the prefix once per row (kernels/attention.cu:57-98); the general kernel of this package does
 // the same, and a 32,767-token prompt in portions of 512 took it 5.5 s at the reference's sizes.  Here a block
 // takes 64 consecutive rows of one (segment, head): keys and values go through shared memory once per 64 rows, in
 // tiles of 32 keys (the second kernel: 64) gathered page by page through the block table by cp.async, the next tile on its
-// way while this one is worked on, the tile after that already looked up in the block table.  Everything is 32-bit
-// arithmetic; the softmax is the online form with running maximum and sum per row (kernels/attention.cu:74-95).
+// way while this one is worked on, the tile after that already looked up in the block table.  Maxima, weights and sums are
+// 32-bit; the softmax is the online form with running maximum and sum per row (kernels/attention.cu:74-95).
 //
 // The first kernel is bound by the issue of multiply-adds and of loads from shared memory, so a thread works on a square of
 // the tile: 4 rows x 4 keys of the scores and 4 rows x HD / 8 dims of P V; the eight threads of a row combine maximum and
@@ -250,9 +251,13 @@ paged_prefill_f32_kernel(const float* q, int q_ld, const float* kc, const float*
 // scores' accumulators already lie as the next product's operand.  Bound by the tensor cores' legacy path (192 products a
 // warp and tile at head size 32) beside the exponentials and the cutting.
 // 512 rows behind 8,192 keys, 8 heads of 32, with the merge of the chunks: 126 us, where the first kernel took 173 and its
-// multiply-adds alone take 59; behind 30,000 keys 453 and 643; head size 64 behind 4,096 keys 137 and 169; one tile of 13 rows 4.9 and 5.2.
+// multiply-adds alone take 59; behind 30,000 keys 453 and 643; one tile of 13 rows 5.1 and 5.4.  Head size 16 behind 8,192 keys 78 and
+// 113, 48 197 and 262, 64 258 and 335.  Above 64 a block's copies and parts leave an SM room for one, and registers spill: head size
+// 80 behind 8,192 keys 471, the first kernel 445, 96 582 and 502, 128 1,010 and 658.
 // Three blocks an SM at head size 32: four, of 128 registers a thread, gain 3 % behind 8,192 keys and lose a third where there are few tiles.
-// Against 64 bits it is no further off than sums of 32-bit products one by one.
+// Against 64 bits (2-norm, 64 to 30,000 keys) it is 0.7e-7 to 5.7e-7 off, where sums of 32-bit products one by one are 1.0e-7 to 200e-7
+// off; the tests hold it to 1.2 times their error + 3e-8.  Only with scores of twenty and more over few keys is it further off than
+// they are (64 keys: 2.2e-7, they 1.3e-7 to 2.1e-7): the tensor cores cut the addends of a sum off where a multiply-add rounds.
 //
 // A value that is not finite has parts that are no numbers: a tile with one, or with one of 10^18 and more (a row tile, for q),
 // is worked out value by value from the 32-bit copies instead, and the next tile is fetched only then.

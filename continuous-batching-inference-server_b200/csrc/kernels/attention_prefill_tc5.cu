@@ -178,10 +178,9 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// Two 32-bit values an instruction, each with its own rounding; the larger of three; 2^x as the special-function unit gives it
-// (exp2f spends three more instructions on results below 2^-126, which are nothing beside a row's largest, 2^-8 at least).
-// With these a thread's 64 scores take some 250 instructions instead of 520.  Together with the exchange of halves at the end (see
-// there): a prompt of 2,048, 16 heads of 128, 44 -> 36 us; 512 rows behind 512 21.5 -> 17.4; 128 rows 8.9 -> 7.5.
+// The largest of three; 2^x by ex2.approx.ftz, which flushes results below 2^-126 to zero: nothing beside a row's largest, which is at
+// least 1 (the key that set the reference).  Together with two values an instruction (packed.cuh) and the exchange of halves at
+// the end (see there): a prompt of 2,048, 16 heads of 128, 44 -> 36 us; 512 rows behind 512 21.5 -> 17.4; 128 rows 8.9 -> 7.5.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));

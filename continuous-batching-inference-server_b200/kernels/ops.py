@@ -817,8 +817,8 @@ def prefill_key_chunks(row_tiles: int, n_head: int, n_seg: int, max_context: int
 def paged_prefill_f32(q, k_cache, v_cache, block_table, cu_rows, seg_start, out, seg0, n_seg, max_seg_rows,
                       n_head, n_kv_head, head_dim, page_size, scale, window=0, chunks=(1, 0), partial=None,
                       positions=None, row0=0, n_rows=0):
-    """The same attention as ``paged_prefill_bf16`` in true 32-bit (up to head size 64 as products of 32-bit values cut into three
-    bfloat16 parts, else by multiply-adds): a block takes 64 rows of one head and brings keys and values through shared memory once.  Head sizes 16, 32, ... 128, any page size;
+    """The same attention as ``paged_prefill_bf16`` over 32-bit values (up to head size 64 as products of the values cut into three
+    bfloat16 parts, summed in 32-bit by the tensor cores, else by 32-bit multiply-adds): a block takes 64 rows of one head and brings keys and values through shared memory once.  Head sizes 16, 32, ... 128, any page size;
     ``q`` and ``out`` in full row numbering.  ``chunks`` = (n, keys) from ``prefill_key_chunks`` cuts the keys n
     ways (every context of the step below n * keys); ``partial`` then holds ``n_rows * n_head * n * (head_dim + 4)``
     floats, ``positions`` the position of every row, ``row0`` and ``n_rows`` name the rows of these segments."""

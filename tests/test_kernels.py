@@ -568,7 +568,7 @@ def test_prefill_attention_tensor_cores(ops, n_head, n_kv_head, hd, ps, window):
                                                            (8, 8, 32, 16, 0), (2, 1, 16, 3, 0), (3, 3, 48, 16, 21),
                                                            (2, 2, 80, 5, 100), (2, 1, 96, 32, 0), (1, 1, 112, 16, 37)])
 def test_prefill_attention_32_bit_tiled(ops, n_head, n_kv_head, hd, ps, window):
-    """The 32-bit tiled form (64 rows to a block, keys through shared memory in tiles of 32): the cases of the
+    """The 32-bit tiled form (64 rows to a block, keys through shared memory in tiles of 64, above head size 64 of 32): the cases of the
     tensor-core form, page sizes that are no power of two, in a cache whose unused slots hold NaN; it agrees with
     the general kernel (one warp per row) to 32-bit rounding."""
     seg_ctx, seg_rows = [200, 333, 64, 70, 1, 130, 600], [200, 77, 64, 3, 1, 65, 257]

@@ -55,6 +55,39 @@ def test_error_against_64_bits(T, hd, n_head, n_kv_head, size):
     assert e_tiled <= 1.2 * e_general + 3e-8, (e_tiled, e_general)
 
 
+@pytest.mark.parametrize("hd, window", [(16, 0), (32, 0), (32, 1000), (48, 0), (64, 300)])
+@pytest.mark.parametrize("one_sign", [False, True])
+def test_error_behind_a_long_context(hd, window, one_sign):
+    """150 rows behind 8,000 keys, the keys whole and cut into chunks that are merged, also with all of q, k and v of one sign, where
+    sums that the tensor cores cut off would all be cut the same way: the bound of the test above, which the general form's
+    long sums leave far behind, and an absolute one (its rows' 32-bit weights and sums, some 2^-23 of each other)."""
+    g = torch.Generator().manual_seed(hd)
+    q, k, v = (torch.randn(n, 2, hd, generator=g) for n in (150, 8150, 8150))
+    if one_sign:
+        q, k, v = q.abs(), k.abs(), v.abs()
+    v = v + 2.0
+    ref = exact(q, k, v, hd, window)
+    for chunks in ((1, 0), (32, 256), (5, 2048)):
+        tiled, general = run(q, k, v, 2, hd, 16, window, chunks)
+        e_tiled, e_general = ((x.double() - ref).norm() / ref.norm() for x in (tiled, general))
+        assert e_tiled <= min(1.2 * e_general + 3e-8, 8e-7), (chunks, e_tiled, e_general)
+
+
+@pytest.mark.parametrize("T", [64, 150])
+@pytest.mark.parametrize("hd", [16, 32, 48, 64])
+def test_error_with_large_scores(hd, T):
+    """Scores of twenty and more over few keys, where a row's error is that of its largest scores: a sum of head-size products
+    whose addends the tensor cores cut off at 2^-24 of the largest one, sixteen at a time, instead of rounding.  Twice the general
+    form's error."""
+    g = torch.Generator().manual_seed(T + hd)
+    q, k, v = (torch.randn(T, 2, hd, generator=g) for _ in range(3))
+    q, v = q * 6, v + 2.0
+    tiled, general = run(q, k, v, 2, hd, 16)
+    ref = exact(q, k, v, hd)
+    e_tiled, e_general = ((x.double() - ref).norm() / ref.norm() for x in (tiled, general))
+    assert e_tiled <= 2 * e_general + 3e-8, (e_tiled, e_general)
+
+
 @pytest.mark.parametrize("hd", [16, 32, 48, 64])
 @pytest.mark.parametrize("size", [1e-30, 1e-35, 1e-38, 1e-41])
 def test_small_values(hd, size):
