@@ -250,7 +250,7 @@ paged_prefill_f32_kernel(const float* q, int q_ld, const float* kc, const float*
 // 32 bits, are cut once per block into shared memory while the next tile is on its way, and P is cut in registers, where the
 // scores' accumulators already lie as the next product's operand.  Bound by the tensor cores' legacy path (192 products a
 // warp and tile at head size 32) beside the exponentials and the cutting.
-// 512 rows behind 8,192 keys, 8 heads of 32, with the merge of the chunks: 126 us, where the first kernel took 173 and its
+// 512 rows behind 8,192 keys, 8 heads of 32, with the merge of the chunks: 125 us, where the first kernel took 173 and its
 // multiply-adds alone take 59; behind 30,000 keys 453 and 643; one tile of 13 rows 5.1 and 5.4.  Head size 16 behind 8,192 keys 78 and
 // 113, 48 197 and 262, 64 258 and 335.  Above 64 a block's copies and parts leave an SM room for one, and registers spill: head size
 // 80 behind 8,192 keys 471, the first kernel 445, 96 582 and 502, 128 1,010 and 658.
@@ -468,8 +468,15 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[2 * np][e] = first[0][e] + rest[0][e];
-          s[2 * np + 1][e] = first[1][e] + rest[1][e];
+          if constexpr (HD < 64) {      // two sums an instruction (at 64 the pairs of registers would spill)
+            if (e % 2) continue;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              unpack2(add2(pack2(first[i][e], first[i][e + 1]), pack2(rest[i][e], rest[i][e + 1])), s[2 * np + i][e], s[2 * np + i][e + 1]);
+          } else {
+            s[2 * np][e] = first[0][e] + rest[0][e];
+            s[2 * np + 1][e] = first[1][e] + rest[1][e];
+          }
         }
       }
     } else {
@@ -499,7 +506,8 @@ paged_prefill_f32_mma_kernel(const float* q, int q_ld, const float* kc, const fl
           }
       } else {
 #pragma unroll
-        for (int n = 0; n < 8; ++n) s[n][2 * hi] *= scale, s[n][2 * hi + 1] *= scale;
+        for (int n = 0; n < 8; ++n)
+          unpack2(mul2(pack2(s[n][2 * hi], s[n][2 * hi + 1]), pack2(scale, scale)), s[n][2 * hi], s[n][2 * hi + 1]);
       }
       float mx = -INFINITY;
 #pragma unroll
