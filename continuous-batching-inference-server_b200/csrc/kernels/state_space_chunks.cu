@@ -20,6 +20,7 @@
 // which stays in registers between chunks (the accumulators of its own update).  155 KB of shared memory at N = 128: one block
 // an SM; the next chunk's rows arrive by cp.async while this one is worked on.
 #include "common.cuh"
+#include "mma_sync.cuh"
 
 namespace cbis {
 namespace ssm {
@@ -40,29 +41,13 @@ __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s32(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void ldm(uint32_t (&r)[4], const void* smem) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s32(smem)) : "memory");
-}
-__device__ __forceinline__ void ldm_t(uint32_t (&r)[4], const void* smem) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s32(smem)) : "memory");
-}
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // Two neighbouring values into three bfloat16 parts each, `part` elements apart.  (What is infinite has rests that are no numbers: it
 // stays not finite, and so does every sum it enters, which are those it enters in the walk row by row.)
 __device__ __forceinline__ void store_parts(__nv_bfloat16* at, int part, float v0, float v1) {
+  unsigned parts[3];
+  cut3(v0, v1, parts);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
-    *reinterpret_cast<__nv_bfloat162*>(at + i * part) = b;
-    v0 -= __low2float(b);
-    v1 -= __high2float(b);
-  }
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<unsigned*>(at + i * part) = parts[i];
 }
 // Whether one of the eight bfloat16 of a fragment is infinite or no number: 0 times it is no number.
 __device__ __forceinline__ bool not_finite(const uint32_t (&r)[4]) {
@@ -201,13 +186,13 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
 #pragma unroll
         for (int k = 0; k < N; k += 16) {
           uint32_t a[4], b0[4], b1[4];
-          ldm(a, sC + (t0 + (lane & 15)) * NP + k + (lane >> 4) * 8);
-          ldm(b0, sB + (s0 + (lane & 7) + ((lane >> 4) << 3)) * NP + k + ((lane >> 3) & 1) * 8);
-          ldm(b1, sB + (s0 + 16 + (lane & 7) + ((lane >> 4) << 3)) * NP + k + ((lane >> 3) & 1) * 8);
-          mma(acc[0], a, b0[0], b0[1]);
-          mma(acc[1], a, b0[2], b0[3]);
-          mma(acc[2], a, b1[0], b1[1]);
-          mma(acc[3], a, b1[2], b1[3]);
+          ldm4<false>(a, sC + (t0 + (lane & 15)) * NP + k + (lane >> 4) * 8);
+          ldm4<false>(b0, sB + (s0 + (lane & 7) + ((lane >> 4) << 3)) * NP + k + ((lane >> 3) & 1) * 8);
+          ldm4<false>(b1, sB + (s0 + 16 + (lane & 7) + ((lane >> 4) << 3)) * NP + k + ((lane >> 3) & 1) * 8);
+          mma_16816(acc[0], a, b0[0], b0[1]);
+          mma_16816(acc[1], a, b0[2], b0[3]);
+          mma_16816(acc[2], a, b1[0], b1[1]);
+          mma_16816(acc[3], a, b1[2], b1[3]);
         }
       }
 #pragma unroll
@@ -243,12 +228,12 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
 #pragma unroll
     for (int k = 0; k < N; k += 16) {
       uint32_t a[4], b[4];
-      ldm(a, sC + (t0 + (lane & 15)) * NP + k + (lane >> 4) * 8);
+      ldm4<false>(a, sC + (t0 + (lane & 15)) * NP + k + (lane >> 4) * 8);
 #pragma unroll
       for (int part = 0; part < 3; ++part) {
-        ldm_t(b, sm + T::S0 + part * N * XP + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + py + (lane >> 4) * 8);
-        mma(part == 0 ? first[0] : rest[0], a, b[0], b[1]);
-        mma(part == 0 ? first[1] : rest[1], a, b[2], b[3]);
+        ldm4<true>(b, sm + T::S0 + part * N * XP + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + py + (lane >> 4) * 8);
+        mma_16816(part == 0 ? first[0] : rest[0], a, b[0], b[1]);
+        mma_16816(part == 0 ? first[1] : rest[1], a, b[2], b[3]);
       }
     }
     {
@@ -263,7 +248,7 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
     // ---- ... then the chunk's own rows, up to the diagonal
     for (int k = 0; k <= t0; k += 16) {
       uint32_t a[4], b[4];
-      ldm_t(b, sX + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + py + (lane >> 4) * 8);
+      ldm4<true>(b, sX + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + py + (lane >> 4) * 8);
       if (k == t0 && __any_sync(0xffffffffu, not_finite(b))) {
         // the zeros above the diagonal times an infinite x of a later row would be no number: these rows one by one, to their own
         for (int s1 = 0; s1 < 16; ++s1)
@@ -280,9 +265,9 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
       }
 #pragma unroll
       for (int part = 0; part < 3; ++part) {
-        ldm(a, sm + T::M0 + part * Q * MP + (t0 + (lane & 15)) * MP + k + (lane >> 4) * 8);
-        mma(part == 0 ? first[0] : rest[0], a, b[0], b[1]);
-        mma(part == 0 ? first[1] : rest[1], a, b[2], b[3]);
+        ldm4<false>(a, sm + T::M0 + part * Q * MP + (t0 + (lane & 15)) * MP + k + (lane >> 4) * 8);
+        mma_16816(part == 0 ? first[0] : rest[0], a, b[0], b[1]);
+        mma_16816(part == 0 ? first[1] : rest[1], a, b[2], b[3]);
       }
     }
 #pragma unroll
@@ -310,15 +295,15 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
 #pragma unroll
     for (int k = 0; k < Q; k += 16) {
       uint32_t a[4];      // B^T: rows of the state, from [s][n]
-      ldm_t(a, sB + (k + (lane & 7) + (lane >> 4) * 8) * NP + n0 + ((lane >> 3) & 1) * 8);
+      ldm4<true>(a, sB + (k + (lane & 7) + (lane >> 4) * 8) * NP + n0 + ((lane >> 3) & 1) * 8);
 #pragma unroll
       for (int part = 0; part < 3; ++part)
 #pragma unroll
         for (int j = 0; j < S_TILES; j += 2) {
           uint32_t b[4];
-          ldm_t(b, sm + T::W0 + part * Q * XP + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + p0 + 8 * j + (lane >> 4) * 8);
-          mma(part == 0 ? s_first[j] : s_rest[j], a, b[0], b[1]);
-          mma(part == 0 ? s_first[j + 1] : s_rest[j + 1], a, b[2], b[3]);
+          ldm4<true>(b, sm + T::W0 + part * Q * XP + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * XP + p0 + 8 * j + (lane >> 4) * 8);
+          mma_16816(part == 0 ? s_first[j] : s_rest[j], a, b[0], b[1]);
+          mma_16816(part == 0 ? s_first[j + 1] : s_rest[j + 1], a, b[2], b[3]);
         }
     }
 #pragma unroll
