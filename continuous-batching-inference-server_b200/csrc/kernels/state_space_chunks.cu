@@ -41,6 +41,9 @@ __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s32(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
+// All nine warps, from two places of the code: a barrier with its number of threads, since __syncthreads() has to be the same
+// call for a whole block.
+__device__ __forceinline__ void block_meets() { asm volatile("barrier.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 // Two neighbouring values into three bfloat16 parts each, `part` elements apart.  (What is infinite has rests that are no numbers: it
 // stays not finite, and so does every sum it enters, which are those it enters in the walk row by row.)
 __device__ __forceinline__ void store_parts(__nv_bfloat16* at, int part, float v0, float v1) {
@@ -141,10 +144,10 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
     scalars(0);
     if (n_chunks > 1) load_raw(1);
     for (int c = 0; c < n_chunks; ++c) {      // the two meetings of every chunk, see below
-      __syncthreads();
+      block_meets();
       if (c + 1 < n_chunks) scalars(c + 1);
       if (c + 2 < n_chunks) load_raw(c + 2);
-      __syncthreads();
+      block_meets();
     }
     return;
   }
@@ -166,7 +169,7 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
   for (int c = 0; c < n_chunks; ++c) {
     const __nv_bfloat16 *sC = sm + T::C0 + (c & 1) * Q * NP, *sB = sm + T::B0 + (c & 1) * Q * NP, *sX = sm + T::X0 + (c & 1) * Q * XP;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();      // the chunk's rows and scalars are there; everyone is done with the chunk before
+    block_meets();      // the chunk's rows and scalars are there; everyone is done with the chunk before
     if (c + 1 < n_chunks) load(c + 1);
     const double* cum = cum2 + (c & 1) * Q;
     const float *dts = dts2 + (c & 1) * Q, *ecum = ecum2 + (c & 1) * Q, *weight = weight2 + (c & 1) * Q;
@@ -214,7 +217,7 @@ ssm_chunks_kernel(const __nv_bfloat16* xbc, int xbc_ld, const __nv_bfloat16* pro
       const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sX + r * XP + p));
       store_parts(sm + T::W0 + r * XP + p, Q * XP, weight[r] * x.x, weight[r] * x.y);
     }
-    __syncthreads();      // the parts of the scores, of the state and of the weighted x are there
+    block_meets();      // the parts of the scores, of the state and of the weighted x are there
     // ---- y of 16 rows and 16 columns: first C S from the state before the chunk, then its decay
     float yv[2][4], first[2][4], rest[2][4];
     auto zero = [&]() {
