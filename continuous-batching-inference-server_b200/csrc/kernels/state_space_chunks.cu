@@ -5,7 +5,7 @@
 //   S'  = e^(c_last) S  +  sum over s of B_s (e^(c_last - c_s) dt_s x_s)^T
 // which is what the row-by-row walk computes, in other groups of sums.  The walk is a chain of dependent steps (422 us for
 // 1,500 rows of 64 heads of 64 x 128 on one prompt, a quarter of a microsecond a row, with most of the SM waiting); here
-// the chain is one step per 64 rows, and the same prompt takes 111 us.  Against 64 bits the results are three times as close as
+// the chain is one step per 64 rows, and the same prompt takes 110 us.  Against 64 bits the results are three times as close as
 // the walk's (2.9e-7 of the largest value, the walk 8.8e-7, over segments of 33 to 700 rows).
 //
 // The products run on the tensor cores (mma.sync m16n8k16, 32-bit sums) without giving up 32-bit values: x, B and C are
@@ -16,7 +16,7 @@
 // was there with a rounding of its own, so that few of these cuts fall on a large value.
 //
 // grid (P / 32, heads, segments), eight warps and one that works out the next chunk's step sizes and decays (a chain of logarithms,
-// exponentials and shuffles in which the eight would wait: 128 us instead of 111, and 115 instead of 86 for 32 heads of 64 x 64): a block walks the chunks of one segment for 32 columns of one head's state,
+// exponentials and shuffles in which the eight would wait: 128 us instead of 110, and 115 instead of 85 for 32 heads of 64 x 64): a block walks the chunks of one segment for 32 columns of one head's state,
 // which stays in registers between chunks (the accumulators of its own update).  155 KB of shared memory at N = 128: one block
 // an SM; the next chunk's rows arrive by cp.async while this one is worked on.
 #include "common.cuh"
