@@ -283,8 +283,11 @@ paged_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int* bt = block_table + (size_t)seg * max_blocks;
 
   // keys and values of rows that no copy will fill must be finite: P is zero there, and 0 * NaN is NaN (only in the stages in use)
-  for (int i = threadIdx.x; i < min(n_tiles, STAGES) * KV_BYTES / 16; i += THREADS)
-    reinterpret_cast<uint4*>(sK)[i] = reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s)
+    if (s == 0 || n_tiles > s)
+      for (int i = s * KV_BYTES / 16 + threadIdx.x; i < (s + 1) * KV_BYTES / 16; i += THREADS)
+        reinterpret_cast<uint4*>(sK)[i] = reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
 
   if (threadIdx.x == 0) {
     bar_init(q_full, 1);
